@@ -1,0 +1,59 @@
+"""The launch forms that depend on the number of particles give the bits of
+each other: a scene alone (few particles) against the same scene inside a
+batch that is past the size where the forms change."""
+import numpy as np
+import pytest
+
+import zsph_b200 as z
+from oracle import pyoracle as po
+from zsph_b200 import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _crowded(n, seed):
+    """A cloud whose densest particles have more neighbours than a list holds."""
+    c = cases.random_cloud(n, seed)
+    rng = np.random.default_rng(seed)
+    mid = c.state.pos.mean(0)
+    k = n // 3
+    c.state.pos[:k] = mid + (c.state.pos[:k] - mid) * 0.2
+    c.state.tmp_pos[:] = c.state.pos
+    c.state.type[:n:7] = 0
+    return c, rng
+
+
+def test_forms_match_across_sizes():
+    small, big = cases.dam_break(0.04), cases.dam_break(0.0135)
+    b = z.Solver.from_batch([small, big, small])
+    assert small.n < 100000 and b.n > 300000
+    b.run(3)
+    got = b.download("old")
+    assert b.status() == 0
+    off = 0
+    for c in (small, big, small):
+        s = z.Solver.from_case(c)
+        s.run(3)
+        want = s.download("old")
+        for k in ("pos", "vel", "rhop", "type", "table"):
+            assert np.array_equal(getattr(got, k)[off:off + c.n], getattr(want, k)), (c.name, k)
+        off += c.n
+        s.close()
+    b.close()
+
+
+def test_walls_with_overflowed_lists():
+    """Lists past their capacity: the pair passes filter the rows again.  The
+    bound is the kernel tests' 1e-4 of the field's scale."""
+    c, _ = _crowded(4001, 5)
+    sol = z.Solver.from_case(c)
+    sol.neighbor_search("old", "new")
+    sol.boundary("new")
+    assert sol.status() & z.FLAG_NB_OVERFLOW
+    o = po.Oracle(c.json, c.state, np.float32)
+    o.search()
+    o.boundary("new")
+    new, want = sol.download("new").rhop, o.new["rhop"]
+    for a in range(2):
+        assert np.abs(new[:, a] - want[:, a]).max() <= 1e-4 * max(np.abs(want[:, a]).max(), 1e-30)
+    sol.close()

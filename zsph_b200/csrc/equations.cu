@@ -339,17 +339,6 @@ __device__ __forceinline__ void wall_term_core(const KParams& kp, float4 pi, flo
   wsum += w;
 }
 
-// Wall pressure contribution of fluid neighbour j of wall particle i
-// (delta_ns.cu:67-85), from j's packed record (one 256-bit load; the sign of
-// its density marks a non-fluid particle).
-template <bool PRECISE = false>
-__device__ __forceinline__ void wall_term(const KParams& kp, const Scratch& s, float4 pi, int j, float& rsum,
-                                          float& wsum, int3 ci = int3{0, 0, 0}) {
-  const ShadowRec r = shadow_rec<PRECISE>(kp, s, j, ci);
-  if (!fluid_of(r.pr.w)) return;
-  wall_term_core(kp, pi, r.pr, make_float2(r.pr.w, r.vp.w), rsum, wsum);
-}
-
 // Particle j's position from the sorted arrays, in the precision form moved
 // into the frame of cell ci (the list build reads the arrays: it writes the
 // packed records itself).
@@ -357,14 +346,6 @@ template <bool PRECISE>
 __device__ __forceinline__ float4 ptc_xyz(const KParams& kp, const zsph_ptc_t& ptc, int j, int3 ci) {
   const float4 p = make_float4(ptc.pos[3 * j], ptc.pos[3 * j + 1], ptc.pos[3 * j + 2], 0.0f);
   return PRECISE ? shifted(kp, p, kp.c3n[j], ci) : p;
-}
-
-// wall_term with the fluid neighbour's data from the sorted arrays
-template <bool PRECISE = false>
-__device__ __forceinline__ void wall_term_ptc(const KParams& kp, const zsph_ptc_t& ptc, float4 pi, int j,
-                                              float& rsum, float& wsum, int3 ci = int3{0, 0, 0}) {
-  if (ptc.type[j] != 1) return;
-  wall_term_core(kp, pi, ptc_xyz<PRECISE>(kp, ptc, j, ci), reinterpret_cast<const float2*>(ptc.rhop)[j], rsum, wsum);
 }
 
 using u64 = unsigned long long;
@@ -417,6 +398,20 @@ __device__ __forceinline__ bool walls_fluid_near(const KParams& kp, const Scratc
   return any;
 }
 
+// Appends particle i to the wall list s.wl where `wall` (one atomic per warp).
+// Every active lane of the warp calls it together.
+__device__ __forceinline__ void append_walls(const KParams& kp, const Scratch& s, int i, bool wall) {
+  const unsigned m = __activemask();
+  const unsigned wm = __ballot_sync(m, wall);
+  if (!wm) return;
+  const int leader = __ffs(m) - 1;
+  int base = 0;
+  if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&s.misc[kMiscWalls], __popc(wm));
+  base = __shfl_sync(m, base, leader);
+  const int slot = base + __popc(wm & lanemask_lt());
+  if (wall && slot < kp.n) s.wl[slot] = i;
+}
+
 // The end of particle i's list build, once s.nb holds its finished list
 // (cnt entries, or ovf): the particle's packed shadow record and list
 // count, and, for a non-fluid particle that can have a fluid neighbour in
@@ -438,17 +433,7 @@ __device__ __forceinline__ void list_tail(const KParams& kp, const Scratch& s, c
   st_rec(&s.sh.pr(i), pr, vp);
   s.nb_cnt[i] = ovf ? kOverflow : (uint8_t)cnt;
   if (ovf) atomicOr(s.flags, ZSPH_FLAG_NB_OVERFLOW);  // rare: the walks re-filter this particle's rows
-  const unsigned m = __activemask();
-  const bool wall = nonfluid && fluid_nb;
-  const unsigned wm = __ballot_sync(m, wall);
-  if (wm) {  // one atomic per warp
-    const int leader = __ffs(m) - 1;
-    int base = 0;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&s.misc[kMiscWalls], __popc(wm));
-    base = __shfl_sync(m, base, leader);
-    const int slot = base + __popc(wm & lanemask_lt());
-    if (wall && slot < kp.n) s.wl[slot] = i;
-  }
+  append_walls(kp, s, i, nonfluid && fluid_nb);
 }
 
 
@@ -727,50 +712,174 @@ template <int GF> struct PairSmem {
 
 // The walls' (rho, p) after the list build (delta_ns.cu:61-85, :116-131):
 // non-fluid particle i extrapolates from the fluid neighbours of its
-// boundary rows, summed in list order, and rewrites the (rho, p) of its
-// packed record (its density stays negative, non-fluid).  The list build has
-// written every record by then, so each neighbour costs one 256-bit load
-// (four ahead of the arithmetic, as in the pair walks), and no fluid record
-// read here is written.  A particle whose list overflowed re-filters its
-// boundary rows.
-template <int GF, bool PRECISE, bool BATCH>
-__device__ __forceinline__ void walls_one(const KParams& kp_arg, const Scratch& s, const zsph_tmp_t& t, int i,
-                                          const PairSmem<GF>& sm) {
-  KParams kp_scene;  // batched form: the parameters of the particle's scene
-  if constexpr (BATCH) kp_scene = kp_of_particle(kp_arg, i);
-  const KParams& kp = BATCH ? kp_scene : kp_arg;
-  const ShadowRec own = s.sh.load(i);
-  const float4 pi = own.pr;
+// boundary rows and rewrites the (rho, p) of its packed record (its density
+// stays negative, non-fluid).  The list build has written every record by
+// then, so each neighbour costs one 256-bit load, and no fluid record read
+// here is written.
+//
+// The sums keep eight partial sums, entry k of the list going to number
+// k % 8, and add them by a fixed tree, so 8 lanes of one partial sum each or
+// 2 of four give the same bits, whatever the size.  At few walls the pass is
+// bound by a wall's chain of dependent loads (list entry -> record): one
+// thread per wall took 26 / 27 / 28 us at 20 k / 105 k / 270 k particles
+// (dam break), 8 lanes take 9 / 10 / 18 and 2 lanes 17 / 18 / 19.  At many
+// walls it is bound by the instructions, to which lanes add row starts and
+// shuffles: one thread, 8 and 2 lanes take 74, 110 and 72 us at 4.2 M, 70, 90
+// and 64 us for 24 scenes of 0.98 M together.  Hence 8 lanes up to kWallsFew
+// particles, 2 beyond.  Eight resident CTAs (64 registers): 2 lanes took
+// 83 us at 4.2 M with 80.
+constexpr int kWallsFew = 300000;
+
+// This thread's partial sums of wall i (lane q of its LANES lanes).  rs: row
+// starts, row r at rs[r * stride].  CY: the list was built at an earlier
+// state, so every entry is tested again and its boundary row decided by the
+// current cells.  A wall whose list overflowed re-filters its rows, candidate
+// k of them all counting as entry k.
+template <int GF, bool PRECISE, bool CY, int LANES>
+__device__ __forceinline__ void wall_sums(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, int i, int q,
+                                          const int* rs, int stride, float4 pi, float (&rsum)[8 / LANES],
+                                          float (&wsum)[8 / LANES]) {
+  constexpr int A = 8 / LANES;         // partial sums of this thread: numbers q * A .. q * A + A - 1
+  constexpr int D = A < 4 ? 4 / A : 1; // 8-entry blocks in flight
   const int3 ci = PRECISE ? unpack_cell(kp.c3n[i]) : int3{0, 0, 0};
-  load_rows<GF>(kp, t, t.hash[i], sm.rs, sm.re);
-  float rsum = 0.0f, wsum = 0.0f;
-  walk<GF, true, NbB1, PRECISE>(
-      kp, s, i, pi, sm.rs, sm.re, sm.rs, i, kp.n - 1,
-      [&](int q) {
-        const ShadowRec r = shadow_rec<PRECISE>(kp, s, q, ci);
-        return NbB1{r.pr, r.vp};
-      },
-      [&](const NbB1& nb) {
-        if (fluid_of(nb.pr.w)) wall_term_core(kp, pi, nb.pr, make_float2(nb.pr.w, nb.vp.w), rsum, wsum);
-      },
-      ci);
-  const zsph_gpu_param_t& p = kp.p;
-  if (fabsf(wsum) > 1e-8f) rsum = rsum / wsum; else rsum = 0.0f;
-  if (rsum < 0.0f) rsum = 0.0f;
-  float4 pr = own.pr, vp = own.vp;
-  pr.w = -(rsum / p.cs2 + p.rho0);  // still non-fluid
-  vp.w = rsum;
-  st_rec(&s.sh.pr(i), pr, vp);
+  const int cy_i = CY ? kp.cur_cy[i] : 0;
+  auto term = [&](int j, ShadowRec o, int cy, bool test, float& rs_, float& ws_) {
+    if (!fluid_of(o.pr.w)) return;
+    if (PRECISE) o.pr = shifted(kp, o.pr, kp.c3n[j], ci);
+    if ((CY || test) && !interacts(kp, dist2(pi.x - o.pr.x, pi.y - o.pr.y, pi.z - o.pr.z))) return;
+    if (CY && (cy - cy_i < -GF || cy - cy_i >= GF)) return;
+    wall_term_core(kp, pi, o.pr, make_float2(o.pr.w, o.vp.w), rs_, ws_);
+  };
+  const int cnt = s.nb_cnt[i];
+  if (cnt != kOverflow) {
+    for (int b = 0; 8 * b < cnt; b += D) {
+#pragma unroll
+      for (int h = 0; h < A; h += 4) {  // at most four entries of a block in flight
+        constexpr int H = A < 4 ? A : 4;
+        int js[D][H], cy[D][H];
+        ShadowRec nb[D][H];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const int k0 = 8 * (b + d) + q * A + h;
+          unsigned w[2] = {0u, 0u};
+          if (k0 < cnt) {
+            const uint16_t* p = s.nb + nb_vec(i, b + d) * 8 + q * A + h;
+            if constexpr (H == 4) {
+              const uint2 v = *reinterpret_cast<const uint2*>(p);
+              w[0] = v.x;
+              w[1] = v.y;
+            } else if constexpr (H == 2) {
+              w[0] = *reinterpret_cast<const unsigned*>(p);
+            } else {
+              w[0] = *p;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < H; ++e) {
+            const unsigned ent = (w[e >> 1] >> ((e & 1) * 16)) & 0xffffu;
+            const int r = (int)(ent >> kRowShift);
+            const bool ok = k0 + e < cnt && (CY || Stencil<GF>::boundary_row(r));
+            js[d][e] = ok ? min(rs[r * stride] + (int)(ent & kOffMask), kp.n - 1) : -1;
+          }
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int e = 0; e < H; ++e) {
+            nb[d][e] = s.sh.load_if(js[d][e] >= 0, js[d][e]);
+            cy[d][e] = CY && js[d][e] >= 0 ? kp.cur_cy[js[d][e]] : 0;
+          }
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int e = 0; e < H; ++e)
+            if (js[d][e] >= 0) term(js[d][e], nb[d][e], cy[d][e], false, rsum[h + e], wsum[h + e]);
+      }
+    }
+    return;
+  }
+  const int c = t.hash[i];
+  int k = 0;  // candidates of the earlier rows
+  for (int r = 0; r < Stencil<GF>::NR; ++r) {
+    if (!CY && !Stencil<GF>::boundary_row(r)) continue;
+    int a, b;
+    row_range<GF>(kp, t, c, r, a, b);
+    for (int j = a; j < b; ++j, ++k) {
+#pragma unroll
+      for (int e = 0; e < A; ++e)
+        if ((k & 7) == q * A + e && j != i) term(j, s.sh.load(j), CY ? kp.cur_cy[j] : 0, true, rsum[e], wsum[e]);
+    }
+  }
 }
 
-// The wall pass over the slots the list build listed in s.wl (grid-stride).
-template <int GF, bool PRECISE = false, bool BATCH = false>
-__global__ void __launch_bounds__(kPairBlock) k_walls(KParams kp, Scratch s, zsph_tmp_t t) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  const PairSmem<GF> sm(dsm);
-  const int nw = min(s.misc[kMiscWalls], kp.n);
-  for (int q = blockIdx.x * kPairBlock + threadIdx.x; q < nw; q += gridDim.x * kPairBlock)
-    walls_one<GF, PRECISE, BATCH>(kp, s, t, s.wl[q], sm);
+// the eight partial sums added: number e with e ^ 4, then e ^ 2, then e ^ 1
+// (every lane of the warp calls it)
+template <int LANES>
+__device__ __forceinline__ float wall_tree(float (&v)[8 / LANES]) {
+  constexpr int A = 8 / LANES;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    if (o >= A) {
+#pragma unroll
+      for (int e = 0; e < A; ++e) v[e] += __shfl_xor_sync(0xffffffffu, v[e], o / A);
+    } else {
+#pragma unroll
+      for (int e = 0; e < o; ++e) v[e] += v[e + o];
+    }
+  }
+  return v[0];
+}
+
+// The walls listed in s.wl by block `blk` of `nblk` blocks of kPairBlock
+// threads (thread `tid` of it), LANES to a wall; s_rs: kPairBlock / LANES * NR
+// ints of the block.
+template <int GF, bool PRECISE, bool BATCH, bool CY, int LANES>
+__device__ __forceinline__ void walls_block(const KParams& kp_arg, const Scratch& s, const zsph_tmp_t& t,
+                                            const zsph_ptc_t* rhop_out, int blk, int nblk, int tid, int* s_rs) {
+  constexpr int NR = Stencil<GF>::NR, W = kPairBlock / LANES, A = 8 / LANES;
+  const int nw = min(s.misc[kMiscWalls], kp_arg.n), g = tid / LANES, q = tid % LANES;
+  int* rs = s_rs + g;
+  for (int w0 = blk * W; w0 < nw; w0 += nblk * W) {  // uniform per block
+    const bool act = w0 + g < nw;
+    const int i = act ? s.wl[w0 + g] : 0;
+    KParams kp_scene;  // batched form: the parameters of the particle's scene
+    if constexpr (BATCH) kp_scene = kp_of_particle(kp_arg, i);
+    const KParams& kp = BATCH ? kp_scene : kp_arg;
+    float rsum[A], wsum[A];
+#pragma unroll
+    for (int e = 0; e < A; ++e) rsum[e] = wsum[e] = 0.0f;
+    ShadowRec own;
+    if (LANES > 1) __syncwarp();  // the previous walls' row starts are no longer read
+    if (act) {
+      own = s.sh.load(i);
+      const int c = t.hash[i];
+#pragma unroll
+      for (int r = q; r < NR; r += LANES) {
+        int e;
+        row_range<GF>(kp, t, c, r, rs[r * W], e);
+      }
+    }
+    if (LANES > 1) __syncwarp();
+    if (act) wall_sums<GF, PRECISE, CY, LANES>(kp, s, t, i, q, rs, W, own.pr, rsum, wsum);
+    float rt = wall_tree<LANES>(rsum);
+    const float wt = wall_tree<LANES>(wsum);
+    if (!act || q != 0) continue;
+    const zsph_gpu_param_t& p = kp.p;
+    if (fabsf(wt) > 1e-8f) rt = rt / wt; else rt = 0.0f;
+    if (rt < 0.0f) rt = 0.0f;
+    const float rho = rt / p.cs2 + p.rho0;
+    float4 pr = own.pr, vp = own.vp;
+    pr.w = -rho;  // still non-fluid
+    vp.w = rt;
+    st_rec(&s.sh.pr(i), pr, vp);
+    if (CY && rhop_out) reinterpret_cast<float2*>(rhop_out->rhop)[i] = make_float2(rho, rt);
+  }
+}
+
+template <int GF, bool PRECISE, bool BATCH, int LANES>
+__global__ void __launch_bounds__(kPairBlock, 8) k_walls(KParams kp, Scratch s, zsph_tmp_t t) {
+  __shared__ int s_rs[kPairBlock / LANES * Stencil<GF>::NR];
+  walls_block<GF, PRECISE, BATCH, false, LANES>(kp, s, t, nullptr, blockIdx.x, gridDim.x, threadIdx.x, s_rs);
 }
 
 // cuda_boundary_ns main part (delta_ns.cu:35-174): renormalisation matrix and
@@ -1216,17 +1325,22 @@ void launch_governing_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_
   }
 }
 
-// The wall pass: enough CTAs to fill the device, each looping over s.wl
-// (its length is known on the device only).
-template <int GF, bool PRECISE = false, bool BATCH = false>
-void launch_walls(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, cudaStream_t st) {
+// CTAs of a wall pass with `lanes` lanes per wall: enough to fill the device,
+// each looping over s.wl (its length is known on the device only).
+inline int walls_grid(int n, int lanes) {
   static int sms = 0;  // SMs of the device (the same for every B200)
   if (!sms) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       sms = 148;
   }
-  k_walls<GF, PRECISE, BATCH><<<min(thread_blocks(kp.n), sms * 16), kPairBlock, pair_smem<GF>(0, 0), st>>>(kp, s, t);
+  const int per_cta = kPairBlock / lanes;
+  return min((n + per_cta - 1) / per_cta, sms * 16);
+}
+template <int GF, bool PRECISE = false, bool BATCH = false>
+void launch_walls(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, cudaStream_t st) {
+  if (kp.n <= kWallsFew) k_walls<GF, PRECISE, BATCH, 8><<<walls_grid(kp.n, 8), kPairBlock, 0, st>>>(kp, s, t);
+  else k_walls<GF, PRECISE, BATCH, 2><<<walls_grid(kp.n, 2), kPairBlock, 0, st>>>(kp, s, t);
 }
 
 // zeroes the wall-list length before a list build appends to it
@@ -1361,55 +1475,24 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
 // otherwise write it).
 //
 // k_cur_cells: each particle's y cell index at its current position, with
-// the hash's arithmetic (hash.cu:13).
-__global__ void __launch_bounds__(kSearchBlock) k_cur_cells(KParams kp, zsph_ptc_t ptc, int* cy) {
+// the hash's arithmetic (hash.cu:13); the non-fluid particles are appended to
+// s.wl (its length zeroed before).
+__global__ void __launch_bounds__(kSearchBlock) k_cur_cells(KParams kp, Scratch s, zsph_ptc_t ptc, int* cy) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kp.n) return;
-  cy[i] = (int)floorf(__fdiv_rn(__fsub_rn(ptc.pos[3 * i + 1], kp.p.grid_ymin), kp.p.grid_size));
+  const bool act = i < kp.n;
+  if (act) cy[i] = (int)floorf(__fdiv_rn(__fsub_rn(ptc.pos[3 * i + 1], kp.p.grid_ymin), kp.p.grid_size));
+  append_walls(kp, s, i, act && ptc.type[i] != 1);
 }
 
-template <int GF>
-__global__ void __launch_bounds__(kPairBlock) k_walls_reuse(KParams kp, Scratch s, zsph_ptc_t ptc, zsph_tmp_t t,
-                                                            int write_rhop) {
-  const int i = blockIdx.x * kPairBlock + threadIdx.x;
-  if (i >= kp.n) return;
-  const float4 pi = s.sh.pr(i);
-  if (fluid_of(pi.w)) return;
-  const int c = t.hash[i];
-  const int cnt = s.nb_cnt[i];
-  const int cy_i = kp.cur_cy[i];
-  float rsum = 0.0f, wsum = 0.0f;
-  auto visit = [&](int j) {
-    const float4 pj = s.sh.pr(j);
-    if (!fluid_of(pj.w) || !interacts(kp, dist2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z))) return;
-    const int row = kp.cur_cy[j] - cy_i;  // the boundary rows by the current cells
-    if (row < -GF || row >= GF) return;
-    wall_term(kp, s, pi, j, rsum, wsum);
-  };
-  if (cnt != kOverflow) {
-    for (int k = 0; k < cnt; ++k) {
-      const unsigned e = s.nb[nb_vec(i, k >> 3) * 8 + (k & 7)];
-      const int r = (int)(e >> kRowShift);
-      int a, b;
-      row_range<GF>(kp, t, c, r, a, b);
-      const int j = a + (int)(e & kOffMask);
-      if (j < b) visit(j);
-    }
-  } else {
-    for (int r = 0; r < Stencil<GF>::NR; ++r) {
-      int a, b;
-      row_range<GF>(kp, t, c, r, a, b);
-      for (int j = a; j < b; ++j)
-        if (j != i) visit(j);
-    }
-  }
-  const zsph_gpu_param_t& p = kp.p;
-  if (fabsf(wsum) > 1e-8f) rsum = rsum / wsum; else rsum = 0.0f;
-  if (rsum < 0.0f) rsum = 0.0f;
-  const float rho = rsum / p.cs2 + p.rho0;
-  s.sh.pr(i).w = -rho;  // still non-fluid
-  s.sh.vp(i).w = rsum;
-  if (write_rhop) reinterpret_cast<float2*>(ptc.rhop)[i] = make_float2(rho, rsum);
+// The walls are those k_cur_cells lists in s.wl.  With one thread per
+// particle, most of them leaving at once, the walls' serial walks took 66 us
+// at 270 k particles; as the wall pass 32 us.
+template <int GF, int LANES>
+__global__ void __launch_bounds__(kPairBlock, 8)
+    k_walls_reuse(KParams kp, Scratch s, zsph_ptc_t ptc, zsph_tmp_t t, int write_rhop) {
+  __shared__ int s_rs[kPairBlock / LANES * Stencil<GF>::NR];
+  walls_block<GF, false, false, true, LANES>(kp, s, t, write_rhop ? &ptc : nullptr, blockIdx.x, gridDim.x,
+                                             threadIdx.x, s_rs);
 }
 
 // Rigid-body contact (see launch_rigid_contact): one thread per particle,
@@ -1620,10 +1703,10 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_batch_persistent(Persist
         nblist_group<1, kPersistWarps, true, false>(kp, s, a.w, a.t, g, wid);
       if (!grid_barrier(a)) return;
       {
-        const int nw = min(s.misc[kMiscWalls], n);
-        const PairSmem<1> sm(dsm + (threadIdx.x / kPairBlock) * pair_smem<1>(0, 0), threadIdx.x % kPairBlock);
-        for (int q = blockIdx.x * kPersistThreads + threadIdx.x; q < nw; q += gridDim.x * kPersistThreads)
-          walls_one<1, false, true>(kp, s, a.t, s.wl[q], sm);
+        const int half = threadIdx.x / kPairBlock;
+        walls_block<1, false, true, false, 2>(kp, s, a.t, nullptr, 2 * blockIdx.x + half, 2 * gridDim.x,
+                                          threadIdx.x % kPairBlock,
+                                          reinterpret_cast<int*>(dsm + half * pair_smem<1>(0, 0)));
       }
       if (!grid_barrier(a)) return;
       persistent_pairs<0>(a, dsm);
@@ -2076,9 +2159,11 @@ cudaError_t launch_corrector_reuse(const KParams& kp_in, const Scratch& s, const
   kp.cur_cy = cy;
   cudaError_t e = launch_pack_shadows(kp, s, ptc, st);
   if (e) return e;
-  k_cur_cells<<<(kp.n + kSearchBlock - 1) / kSearchBlock, kSearchBlock, 0, st>>>(kp, ptc, cy);
+  if ((e = reset_walls(s, st))) return e;
+  k_cur_cells<<<(kp.n + kSearchBlock - 1) / kSearchBlock, kSearchBlock, 0, st>>>(kp, s, ptc, cy);
   const int nb = thread_blocks(kp.n), sm = pair_smem<1>(0, 0);
-  k_walls_reuse<1><<<nb, kPairBlock, 0, st>>>(kp, s, ptc, t, fresh_boundary ? 0 : 1);
+  if (kp.n <= kWallsFew) k_walls_reuse<1, 8><<<walls_grid(kp.n, 8), kPairBlock, 0, st>>>(kp, s, ptc, t, fresh_boundary ? 0 : 1);
+  else k_walls_reuse<1, 2><<<walls_grid(kp.n, 2), kPairBlock, 0, st>>>(kp, s, ptc, t, fresh_boundary ? 0 : 1);
   if (fresh_boundary) k_boundary<1, false, false, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t);
   const FeatOut none{};
   if (mode == 2) k_governing<1, 2, false, false, false, false, 1, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, ptc, none);

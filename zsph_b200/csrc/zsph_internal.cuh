@@ -129,6 +129,13 @@ __device__ __forceinline__ void ld_rec(const float4* p, float4& a, float4& b) {
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
       : "l"(p));
 }
+// ld_rec where `ok`; elsewhere no access is made and a, b are undefined.
+__device__ __forceinline__ void ld_rec_if(bool ok, const float4* p, float4& a, float4& b) {
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
+      "@p ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p), "r"((unsigned)ok));
+}
 __device__ __forceinline__ void st_rec(float4* p, float4 a, float4 b) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
                "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
@@ -154,6 +161,12 @@ struct Shadow {
   __device__ __forceinline__ ShadowRec load(int i) const {
     ShadowRec r;
     ld_rec(rec + 2 * i, r.pr, r.vp);
+    return r;
+  }
+  // the record where `ok`; elsewhere no access is made and the value is undefined
+  __device__ __forceinline__ ShadowRec load_if(bool ok, int i) const {
+    ShadowRec r;
+    ld_rec_if(ok, rec + 2 * i, r.pr, r.vp);
     return r;
   }
 };
