@@ -1,22 +1,21 @@
 // Learned-corrector network on the fifth-generation tensor cores (sm_100a).
 //
 // MLP 32 -> 128 -> 128 -> 4, SiLU, bf16 operands, fp32 accumulation in TMEM.
-// One CTA of 128 threads owns one 128-row tile at a time: thread t <-> tile
-// row t <-> TMEM lane t.  Thread 0 issues tcgen05.mma from shared-memory
-// operands (layout: umma.cuh) and commits to one mbarrier; every thread then
-// reads its row of the accumulator with tcgen05.ld, applies bias and SiLU and
-// writes the next layer's bf16 operand row back to shared memory.
+// A tile is 128 rows: row <-> TMEM lane.  One thread issues tcgen05.mma from
+// shared-memory operands (layout: umma.cuh) and commits to an mbarrier; every
+// thread then reads its row of the accumulator with tcgen05.ld, applies bias
+// and SiLU and writes the next layer's bf16 operand row back to shared memory.
 //
-// Modes of the one kernel:
+// k_mlp_infer<MODE>, four tiles in flight per CTA, one thread per row:
 //   kPredict  standardized outputs per row -> global memory
 //   kCorrect  learned corrector epilogue: acceleration and drho/dt of the
 //             corrector stage = predictor-stage values + de-standardized
 //             network output, then the time_int.cu:50-92 correction in place
-//   kTrain    forward + backward of the weighted squared error; the weight
-//             gradients accumulate in TMEM across all tiles of the CTA
-//             (dW = G^T H with G and H read MN-major from the same buffers
-//             the forward pass wrote K-major) and leave as one partial row
-//             per CTA, reduced deterministically by the Adam kernel.
+// k_mlp_train, one tile per CTA at a time, two threads per row: forward +
+//   backward of the weighted squared error; the weight gradients accumulate
+//   in TMEM across all tiles of the CTA (dW = G^T H with G and H read
+//   MN-major from the same buffers the forward pass wrote K-major) and leave
+//   as one partial row per CTA, reduced deterministically by the Adam kernel.
 // SiLU(z) = z * s(z), s(z) = 0.5 tanh(z/2) + 0.5 with the MUFU tanh; its
 // derivative s (1 + z (1 - s)) is kept as bf16 for the backward pass.
 #include <cuda_bf16.h>
@@ -43,41 +42,51 @@ constexpr int kNPartial = ZSPH_MLP_NPARTIAL;
 static_assert(kNParam == ZSPH_MLP_NPARAM, "parameter layout");
 static_assert(kNPartial >= kNParam + 1 && kNPartial % 4 == 0, "partial row layout");
 
-enum { kPredict = 0, kCorrect = 1, kTrain = 2 };
+enum { kPredict = 0, kCorrect = 1 };
 
-// Shared-memory map (bytes).  Inference reuses the layer-1 activation buffer
-// for layer 2 and needs no backward buffers: 88 KB, two CTAs per SM.
-template <int MODE> struct Smem {
-  static constexpr bool TR = MODE == kTrain;
-  static constexpr uint32_t X = 0;                                 // 128 x 32
-  static constexpr uint32_t H1 = X + 8192;                         // 128 x 128
-  static constexpr uint32_t H2 = TR ? H1 + 32768 : H1;             // 128 x 128
-  static constexpr uint32_t S1 = H2 + 32768;                       // silu'(z1), then G1
-  static constexpr uint32_t S2 = TR ? S1 + 32768 : S1;             // silu'(z2), then G2
-  static constexpr uint32_t G3 = TR ? S2 + 32768 : S2;             // 128 x 16
-  static constexpr uint32_t ONES = TR ? G3 + 4096 : G3;            // 128 x 16, column 0 = 1
-  static constexpr uint32_t W1 = TR ? ONES + 4096 : ONES;          // 128 x 32
-  static constexpr uint32_t W2 = W1 + 8192;                        // 128 x 128
-  static constexpr uint32_t W3 = W2 + 32768;                       // 16 x 128
-  static constexpr uint32_t B = W3 + 4096;                         // b1, b2, b3 (fp32)
-  static constexpr uint32_t CTRL = B + 1088;                       // mbarrier, tmem address, reductions
-  static constexpr uint32_t BYTES = CTRL + 256;
-  // dynamic shared memory requested: more than BYTES so that every operand
-  // span an MMA can address (start + 15 blocks at either byte offset) lies
-  // inside the allocation; inference still fits two CTAs per SM
-  static constexpr uint32_t ALLOC = TR ? 227 * 1024 : 113 * 1024;
-  static constexpr uint32_t NCOLS = TR ? 512 : 256;                // TMEM columns
+// Shared-memory maps (bytes).  Inference: the weights once per CTA, then one
+// X and one activation buffer (layer 2's output over layer 1's) per tile in
+// flight.  More dynamic shared memory is requested than the maps end at, so
+// that every operand span an MMA can address (start + 15 blocks at either
+// byte offset) lies inside the allocation.
+constexpr uint32_t kAlloc = 227 * 1024;
+constexpr int kInferTiles = 4;  // tiles in flight per CTA, 128 threads and 128 TMEM columns each
+struct InferSmem {
+  static constexpr uint32_t W1 = 0;              // 128 x 32
+  static constexpr uint32_t W2 = W1 + 8192;      // 128 x 128
+  static constexpr uint32_t W3 = W2 + 32768;     // 16 x 128
+  static constexpr uint32_t B = W3 + 4096;       // b1 / 2, b2 / 2, b3 (fp32)
+  static constexpr uint32_t CTRL = B + 1088;     // mbarriers, tmem address
+  static constexpr uint32_t TILE = CTRL + 320;   // first tile's buffers
+  static constexpr uint32_t X = 0, H = 8192, TILE_BYTES = 8192 + 32768;
+  static constexpr uint32_t BYTES = TILE + kInferTiles * TILE_BYTES;
 };
-static_assert(Smem<kTrain>::BYTES <= 227 * 1024, "train shared memory");
-static_assert(Smem<kCorrect>::BYTES <= Smem<kCorrect>::ALLOC && Smem<kTrain>::BYTES <= Smem<kTrain>::ALLOC, "");
-static_assert(2 * (Smem<kCorrect>::ALLOC + 1024) <= 228 * 1024, "two inference CTAs per SM");
+static_assert(InferSmem::TILE % 128 == 0 && InferSmem::BYTES + 16384 <= kAlloc, "inference shared memory");
+struct TrainSmem {
+  static constexpr uint32_t X = 0;               // 128 x 32
+  static constexpr uint32_t H1 = X + 8192;       // 128 x 128
+  static constexpr uint32_t H2 = H1 + 32768;     // 128 x 128
+  static constexpr uint32_t S1 = H2 + 32768;     // silu'(z1), then G1
+  static constexpr uint32_t S2 = S1 + 32768;     // silu'(z2), then G2
+  static constexpr uint32_t G3 = S2 + 32768;     // 128 x 16
+  static constexpr uint32_t ONES = G3 + 4096;    // 128 x 16, column 0 = 1
+  static constexpr uint32_t W1 = ONES + 4096;    // 128 x 32
+  static constexpr uint32_t W2 = W1 + 8192;      // 128 x 128
+  static constexpr uint32_t W3 = W2 + 32768;     // 16 x 128
+  static constexpr uint32_t B = W3 + 4096;       // b1, b2, b3 (fp32)
+  static constexpr uint32_t CTRL = B + 1088;     // mbarrier, tmem address, reductions
+  static constexpr uint32_t BYTES = CTRL + 256;
+};
+static_assert(TrainSmem::BYTES <= kAlloc, "train shared memory");
 
-// TMEM column map (fp32 columns; lane = tile row, or output unit for dW)
+// TMEM column map of training (fp32 columns; lane = tile row, or output unit
+// for dW).  Inference gives tile g of a CTA the columns 128 g .. 128 g + 127,
+// z1, z2 and z3 one after another.
 constexpr uint32_t cZ1 = 0;     // z1, later dH2
 constexpr uint32_t cZ2 = 128;   // z2, later dH1
 constexpr uint32_t cDW2 = 256;  // dW2 [out][in]
 constexpr uint32_t cDW1 = 384;  // dW1 [out][in]
-constexpr uint32_t cZ3 = 416;   // z3 (train); inference puts z3 at cZ1
+constexpr uint32_t cZ3 = 416;   // z3
 constexpr uint32_t cDW3 = 432;  // dW3^T [in][out]
 constexpr uint32_t cDB1 = 448;  // db1 in column 0
 constexpr uint32_t cDB2 = 464;  // db2 in column 0
@@ -141,12 +150,69 @@ __device__ void load_operand(unsigned char* dst, const __nv_bfloat16* src, int R
   }
 }
 
-// z = acc + bias -> h = silu(z) (and s = silu'(z) when training), bf16 rows
-template <bool TR>
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {  // each half rounded as fmaf
+  unsigned long long r;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+      "fma.rn.f32x2 %0, a, b, c;\n\t}"
+      : "=l"(r)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+  float2 o;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));
+  return o;
+}
+
+__device__ __forceinline__ float2 mul2(float2 x, float2 y) {  // each half rounded as x * y
+  unsigned long long r;
+  asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\tmul.rn.f32x2 %0, a, b;\n\t}"
+      : "=l"(r)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+  float2 o;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));
+  return o;
+}
+
+// Inference: h = silu(acc + bias) as bf16 rows.  With y = z / 2 and
+// t = tanh(y), silu(z) = y (t + 1); `hbias` holds bias / 2, so
+// y = fma(acc, 1/2, bias/2) rounds as (acc + bias) / 2, and the scalings by
+// two keep every rounding that of z * (t/2 + 1/2).  Per two elements: three
+// packed operations, two MUFU operations and one conversion.  The next
+// 16 columns are on their way from TMEM while these are worked on.
+__device__ __forceinline__ void silu_rows(uint32_t taddr, const float* hbias, unsigned char* sH, int row) {
+  const float2 half = make_float2(0.5f, 0.5f), one = make_float2(1.0f, 1.0f);
+  uint32_t v[2][16];
+  tmem_ld16_start(taddr, v[0]);
+#pragma unroll
+  for (int c = 0; c < kHid / 16; ++c) {
+    uint32_t(&w)[16] = v[c & 1];
+    tmem_ld16_wait(w);
+    if (c + 1 < kHid / 16) tmem_ld16_start(taddr + 16 * (c + 1), v[(c + 1) & 1]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint32_t h[4];
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const int j = q * 8 + 2 * e;
+        const float4 b = *reinterpret_cast<const float4*>(hbias + 16 * c + j);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const float2 a = make_float2(__uint_as_float(w[j + 2 * d]), __uint_as_float(w[j + 2 * d + 1]));
+          const float2 y = fma2(a, half, d ? make_float2(b.z, b.w) : make_float2(b.x, b.y));
+          const float2 t = make_float2(tanh_mufu(y.x), tanh_mufu(y.y));
+          const float2 r = mul2(y, fma2(t, one, one));
+          h[e + d] = pack_bf16(r.x, r.y);
+        }
+      }
+      *reinterpret_cast<uint4*>(sH + core_off(128, row, 16 * c + 8 * q)) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+  }
+}
+
+// Training: z = acc + bias -> h = silu(z) and s = silu'(z), bf16 rows,
+// columns c_lo .. c_lo + kHid / 2 - 1
 __device__ __forceinline__ void hidden_rows(uint32_t taddr, const float* bias, unsigned char* sH, unsigned char* sS,
-                                            int row) {
+                                            int row, int c_lo) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < kHid; c0 += 32) {
+  for (int c0 = c_lo; c0 < c_lo + kHid / 2; c0 += 32) {
     float v[32];
     tmem_ld32(taddr + c0, v);
 #pragma unroll
@@ -155,22 +221,23 @@ __device__ __forceinline__ void hidden_rows(uint32_t taddr, const float* bias, u
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int j = q * 8 + 2 * e;
-        const float z0 = v[j] + bias[c0 + j], z1 = v[j + 1] + bias[c0 + j + 1];
+        const float2 b = *reinterpret_cast<const float2*>(bias + c0 + j);
+        const float z0 = v[j] + b.x, z1 = v[j + 1] + b.y;
         const float s0 = fmaf(0.5f, tanh_mufu(0.5f * z0), 0.5f), s1 = fmaf(0.5f, tanh_mufu(0.5f * z1), 0.5f);
         h[e] = pack_bf16(z0 * s0, z1 * s1);
-        if (TR) s[e] = pack_bf16(s0 * fmaf(z0, 1.0f - s0, 1.0f), s1 * fmaf(z1, 1.0f - s1, 1.0f));
+        s[e] = pack_bf16(s0 * fmaf(z0, 1.0f - s0, 1.0f), s1 * fmaf(z1, 1.0f - s1, 1.0f));
       }
       const uint32_t off = core_off(128, row, c0 + q * 8);
       *reinterpret_cast<uint4*>(sH + off) = make_uint4(h[0], h[1], h[2], h[3]);
-      if (TR) *reinterpret_cast<uint4*>(sS + off) = make_uint4(s[0], s[1], s[2], s[3]);
+      *reinterpret_cast<uint4*>(sS + off) = make_uint4(s[0], s[1], s[2], s[3]);
     }
   }
 }
 
-// G = dH (TMEM) * silu' (bf16 in sS), written over sS
-__device__ __forceinline__ void grad_rows(uint32_t taddr, unsigned char* sS, int row) {
+// G = dH (TMEM) * silu' (bf16 in sS), written over sS; columns as hidden_rows
+__device__ __forceinline__ void grad_rows(uint32_t taddr, unsigned char* sS, int row, int c_lo) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < kHid; c0 += 32) {
+  for (int c0 = c_lo; c0 < c_lo + kHid / 2; c0 += 32) {
     float v[32];
     tmem_ld32(taddr + c0, v);
 #pragma unroll
@@ -190,16 +257,182 @@ __device__ __forceinline__ void grad_rows(uint32_t taddr, unsigned char* sS, int
   }
 }
 
+// N consecutive floats of one thread; al: p is 16-byte aligned
+template <int N>
+__device__ __forceinline__ void store_cols(float* p, const float (&v)[N], bool al) {
+  if (al) {
+#pragma unroll
+    for (int j = 0; j < N; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) p[j] = v[j];
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
+// barrier `id` over the 128 threads of one inference tile
+__device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ bool tile_sync_or(int id, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(id)
+      : "memory");
+  return r != 0;
+}
+
+// Inference (kPredict, kCorrect).  A tile is a chain MMA -> TMEM load -> SiLU
+// -> bf16 store -> next MMA, in which the tensor cores wait for the threads
+// and the threads for the tensor cores; what bounds it with enough tiles in
+// flight is the MUFU tanh (256 per row: some 57 us per million rows).  A CTA
+// therefore keeps kInferTiles independent tiles in flight, 128 threads, one
+// mbarrier, 128 TMEM columns and 40 KB of buffers each, on one copy of the
+// weights (one CTA per SM), and loads a tile's next rows during its first
+// MMA.  With two CTAs of one tile per SM (and one copy of the weights each) a
+// million rows took 141 us; with four, 104 us.
 template <int MODE>
-__global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
-  using L = Smem<MODE>;
-  constexpr bool TR = L::TR;
+__global__ void __launch_bounds__(128 * kInferTiles, 1) k_mlp_infer(MlpArgs a) {
+  using L = InferSmem;
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, lt = tid & 127;
+  unsigned char* sX = sm + L::TILE + g * L::TILE_BYTES + L::X;
+  unsigned char* sH = sm + L::TILE + g * L::TILE_BYTES + L::H;
+  unsigned char* sW1 = sm + L::W1;
+  unsigned char* sW2 = sm + L::W2;
+  unsigned char* sW3 = sm + L::W3;
+  float* sB1 = reinterpret_cast<float*>(sm + L::B);
+  float* sB2 = sB1 + kHid;
+  float* sB3 = sB2 + kHid;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::CTRL) + g;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(sm + L::CTRL + 8 * kInferTiles);
+
+  if (warp == 0) {
+    tmem_alloc(s_tmem, 128 * kInferTiles);
+    tmem_relinquish();
+  }
+  if (lt == 0) mbar_init(bar, 1);
+  int it = blockIdx.x + g * gridDim.x;  // this tile slot's tiles: it, it + kInferTiles * gridDim.x, ...
+  uint4 x[4];
+  auto load_x = [&](int tile) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = a.x[(size_t)tile * 512 + lt + 128 * k];
+  };
+  auto store_x = [&]() {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(sX)[lt + 128 * k] = x[k];
+  };
+  if (it < a.ntiles) load_x(it);
+  load_operand(sW1, a.net.w1, kHid, kIn);
+  load_operand(sW2, a.net.w2, kHid, kHid);
+  load_operand(sW3, a.net.w3p, kOutPad, kHid);
+  if (tid < kHid) {
+    sB1[tid] = 0.5f * a.net.b1[tid];
+    sB2[tid] = 0.5f * a.net.b2[tid];
+  }
+  if (tid < kOut) sB3[tid] = a.net.b3[tid];
+  if (it < a.ntiles) store_x();
+  fence_proxy_async();
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tb = *s_tmem + 128 * g;
+  const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;  // this warp's TMEM lanes
+  const int sync_id = 1 + g;
+
+  uint32_t phase = 0;
+  bool failed = false;
+  // bounded wait for the MMAs committed last; false (on every thread of the tile) if it timed out
+  auto wait_mma = [&]() -> bool {
+    const bool ok = mbar_wait(bar, phase);
+    if (tile_sync_or(sync_id, !ok)) return false;
+    phase ^= 1u;
+    fence_after();
+    return true;
+  };
+  // the threads' shared-memory and TMEM accesses so far, before the MMAs issued next
+  auto before_mma = [&]() {
+    fence_proxy_async();
+    fence_before();
+    tile_sync(sync_id);
+  };
+
+  for (; it < a.ntiles; it += kInferTiles * gridDim.x) {
+    const int row = it * 128 + lt;
+    const int next = it + kInferTiles * gridDim.x;
+    before_mma();
+    if (lt == 0) {
+      fence_after();
+      mma(tb, kmaj(sX, 128, 0), kmaj(sW1, 128, 0), kId128x128KK, false);
+      mma(tb, kmaj(sX, 128, 1), kmaj(sW1, 128, 1), kId128x128KK, true);
+      commit(bar);
+    }
+    if (next < a.ntiles) load_x(next);
+    if (!wait_mma()) { failed = true; break; }
+    if (next < a.ntiles) store_x();  // layer 1 has read the tile's rows
+    silu_rows(tb + lrow, sB1, sH, lt);
+    before_mma();
+    if (lt == 0) {
+      fence_after();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) mma(tb, kmaj(sH, 128, k), kmaj(sW2, 128, k), kId128x128KK, k > 0);
+      commit(bar);
+    }
+    if (!wait_mma()) { failed = true; break; }
+    silu_rows(tb + lrow, sB2, sH, lt);
+    before_mma();
+    if (lt == 0) {
+      fence_after();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) mma(tb, kmaj(sH, 128, k), kmaj(sW3, kOutPad, k), kId128x16KK, k > 0);
+      commit(bar);
+    }
+    if (!wait_mma()) { failed = true; break; }
+    float z3[16];
+    tmem_ld16(tb + lrow, z3);
+    float yh[kOut];
+#pragma unroll
+    for (int k = 0; k < kOut; ++k) yh[k] = z3[k] + sB3[k];
+    if (MODE == kPredict) {
+      if (row < a.nrows) a.out[row] = make_float4(yh[0], yh[1], yh[2], yh[3]);
+    } else if (row < a.nrows && a.ptc.type[row] == 1) {
+      // corrector stage = linear extrapolation a_n + D + learned residual
+      float4 acc = a.acc[row];
+      const float4 d = a.dprev[row];
+      acc.x += d.x + fmaf(yh[0], a.oa.x, a.ob.x);
+      acc.y += d.y + fmaf(yh[1], a.oa.y, a.ob.y);
+      acc.z += d.z + fmaf(yh[2], a.oa.z, a.ob.z);
+      acc.w += d.w + fmaf(yh[3], a.oa.w, a.ob.w);
+      a.acc[row] = acc;
+      if (!isfinite(acc.x + acc.y + acc.z + acc.w)) atomicOr(a.flags, ZSPH_FLAG_NAN);
+      integrate_one<2>(a.kp, a.ptc, a.ptc, row, acc);
+    }
+  }
+  if (failed) {  // report, let the MMAs in flight land (bounded)
+    if (lt == 0) atomicOr(a.flags, ZSPH_FLAG_TIMEOUT);
+    mbar_wait(bar, phase);
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(*s_tmem, 128 * kInferTiles);
+}
+
+// Training: forward, backward and the weight gradients of one batch.  One
+// tile per CTA at a time (the buffers fill the SM), two threads per row: warp
+// w and warp w + 4 share the TMEM lanes of rows 32 (w % 4) .. + 31 and take
+// half of the columns each.  Batches are a tile or two per SM, so a launch is
+// one tile's chain of MMAs and row passes plus the weights' load and the
+// partial gradients' store: 31 us with one thread per row and 4-byte stores of
+// the partial rows, 16.5 us now (148 tiles).
+constexpr int kTrainThreads = 256;
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(MlpArgs a) {
+  using L = TrainSmem;
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* sX = sm + L::X;
   unsigned char* sH1 = sm + L::H1;
@@ -219,30 +452,29 @@ __global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
   float* s_red = reinterpret_cast<float*>(sm + L::CTRL + 16);  // [4 warps][8]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lt = tid & 127, half = tid >> 7;  // row and column half
+  const int c_lo = half * (kHid / 2);
   if (warp == 0) {
-    tmem_alloc(s_tmem, L::NCOLS);
+    tmem_alloc(s_tmem, 512);
     tmem_relinquish();
   }
   if (tid == 0) mbar_init(bar, 1);
   load_operand(sW1, a.net.w1, kHid, kIn);
   load_operand(sW2, a.net.w2, kHid, kHid);
   load_operand(sW3, a.net.w3p, kOutPad, kHid);
-  for (int k = tid; k < kHid; k += 128) {
-    sB1[k] = a.net.b1[k];
-    sB2[k] = a.net.b2[k];
+  if (tid < kHid) {
+    sB1[tid] = a.net.b1[tid];
+    sB2[tid] = a.net.b2[tid];
   }
   if (tid < kOut) sB3[tid] = a.net.b3[tid];
-  if (TR) {
-    // ones operand [128 rows][16]: column 0 = 1.0 (bf16 0x3F80)
-    *reinterpret_cast<uint4*>(sOnes + core_off(128, tid, 0)) = make_uint4(0x3F80u, 0u, 0u, 0u);
-    *reinterpret_cast<uint4*>(sOnes + core_off(128, tid, 8)) = make_uint4(0u, 0u, 0u, 0u);
-  }
+  // ones operand [128 rows][16]: column 0 = 1.0 (bf16 0x3F80)
+  *reinterpret_cast<uint4*>(sOnes + core_off(128, lt, 8 * half)) = make_uint4(half ? 0u : 0x3F80u, 0u, 0u, 0u);
   fence_proxy_async();
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tb = *s_tmem;
-  const uint32_t lrow = (uint32_t)(warp * 32) << 16;  // this warp's TMEM lanes
+  const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;  // this warp's TMEM lanes
 
   uint32_t phase = 0;
   bool failed = false;
@@ -260,10 +492,13 @@ __global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
 
   for (int it = blockIdx.x; it < a.ntiles; it += gridDim.x) {
     const int tile = a.tile_ids ? a.tile_ids[it] : it;
-    const int row = tile * 128 + tid;
+    const int row = tile * 128 + lt;
     const uint4* src = a.x + (size_t)tile * 512;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) reinterpret_cast<uint4*>(sX)[tid + 128 * k] = src[tid + 128 * k];
+    for (int k = 0; k < 2; ++k)
+      reinterpret_cast<uint4*>(sX)[tid + kTrainThreads * k] = src[tid + kTrainThreads * k];
+    const float4 yt = a.y[row];
+    const float w = a.wrow[row];
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
@@ -273,7 +508,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
       commit(bar);
     }
     if (!wait_mma()) { failed = true; break; }
-    hidden_rows<TR>(tb + lrow + cZ1, sB1, sH1, sS1, tid);
+    hidden_rows(tb + lrow + cZ1, sB1, sH1, sS1, lt, c_lo);
     fence_proxy_async();
     fence_before();
     __syncthreads();
@@ -284,135 +519,116 @@ __global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
       commit(bar);
     }
     if (!wait_mma()) { failed = true; break; }
-    hidden_rows<TR>(tb + lrow + cZ2, sB2, sH2, sS2, tid);
+    hidden_rows(tb + lrow + cZ2, sB2, sH2, sS2, lt, c_lo);
     fence_proxy_async();
     fence_before();
     __syncthreads();
-    const uint32_t cz3 = TR ? cZ3 : cZ1;
     if (tid == 0) {
       fence_after();
 #pragma unroll
-      for (int k = 0; k < 8; ++k) mma(tb + cz3, kmaj(sH2, 128, k), kmaj(sW3, kOutPad, k), kId128x16KK, k > 0);
+      for (int k = 0; k < 8; ++k) mma(tb + cZ3, kmaj(sH2, 128, k), kmaj(sW3, kOutPad, k), kId128x16KK, k > 0);
       commit(bar);
     }
     if (!wait_mma()) { failed = true; break; }
-    float z3[16];
-    tmem_ld16(tb + lrow + cz3, z3);
-    float yh[kOut];
-#pragma unroll
-    for (int k = 0; k < kOut; ++k) yh[k] = z3[k] + sB3[k];
-
-    if (MODE == kPredict) {
-      if (row < a.nrows) a.out[row] = make_float4(yh[0], yh[1], yh[2], yh[3]);
-    } else if (MODE == kCorrect) {
-      if (row < a.nrows && a.ptc.type[row] == 1) {
-        // corrector stage = linear extrapolation a_n + D + learned residual
-        float4 acc = a.acc[row];
-        const float4 d = a.dprev[row];
-        acc.x += d.x + fmaf(yh[0], a.oa.x, a.ob.x);
-        acc.y += d.y + fmaf(yh[1], a.oa.y, a.ob.y);
-        acc.z += d.z + fmaf(yh[2], a.oa.z, a.ob.z);
-        acc.w += d.w + fmaf(yh[3], a.oa.w, a.ob.w);
-        a.acc[row] = acc;
-        if (!isfinite(acc.x + acc.y + acc.z + acc.w)) atomicOr(a.flags, ZSPH_FLAG_NAN);
-        integrate_one<2>(a.kp, a.ptc, a.ptc, row, acc);
-      }
-    } else {
+    if (half == 0) {
       // d loss / d yhat, loss and db3 partial sums (fp32, per thread)
-      const float4 yt = a.y[row];
-      const float w = a.wrow[row];
+      float z3[16];
+      tmem_ld16(tb + lrow + cZ3, z3);
       const float yv[kOut] = {yt.x, yt.y, yt.z, yt.w};
       float g[kOut];
 #pragma unroll
       for (int k = 0; k < kOut; ++k) {
-        const float d = yh[k] - yv[k];
+        const float d = z3[k] + sB3[k] - yv[k];
         r_loss = fmaf(w * d, d, r_loss);
         g[k] = 2.0f * w * d * a.inv_wsum;
         r_db3[k] += g[k];
       }
-      *reinterpret_cast<uint4*>(sG3 + core_off(128, tid, 0)) =
+      *reinterpret_cast<uint4*>(sG3 + core_off(128, lt, 0)) =
           make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), 0u, 0u);
-      *reinterpret_cast<uint4*>(sG3 + core_off(128, tid, 8)) = make_uint4(0u, 0u, 0u, 0u);
-      fence_proxy_async();
-      fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        fence_after();
-        // dW3^T[in][out] += H2^T G3 ; dH2 = G3 W3
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          mma(tb + cDW3, mnmaj(sH2, 128, k), mnmaj(sG3, 128, k), kId128x16MM, !(first && k == 0));
-        mma(tb + cZ1, kmaj(sG3, 128, 0), mnmaj(sW3, kOutPad, 0), kId128x128KM, false);
-        commit(bar);
-      }
-      if (!wait_mma()) { failed = true; break; }
-      grad_rows(tb + lrow + cZ1, sS2, tid);  // G2
-      fence_proxy_async();
-      fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        fence_after();
-        // dW2[out][in] += G2^T H1 ; db2 += G2^T 1 ; dH1 = G2 W2
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          mma(tb + cDW2, mnmaj(sS2, 128, k), mnmaj(sH1, 128, k), kId128x128MM, !(first && k == 0));
-          mma(tb + cDB2, mnmaj(sS2, 128, k), mnmaj(sOnes, 128, k), kId128x16MM, !(first && k == 0));
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) mma(tb + cZ2, kmaj(sS2, 128, k), mnmaj(sW2, 128, k), kId128x128KM, k > 0);
-        commit(bar);
-      }
-      if (!wait_mma()) { failed = true; break; }
-      grad_rows(tb + lrow + cZ2, sS1, tid);  // G1
-      fence_proxy_async();
-      fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        fence_after();
-        // dW1[out][in] += G1^T X ; db1 += G1^T 1
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          mma(tb + cDW1, mnmaj(sS1, 128, k), mnmaj(sX, 128, k), kId128x32MM, !(first && k == 0));
-          mma(tb + cDB1, mnmaj(sS1, 128, k), mnmaj(sOnes, 128, k), kId128x16MM, !(first && k == 0));
-        }
-        commit(bar);
-      }
-      if (!wait_mma()) { failed = true; break; }
-      first = false;
+      *reinterpret_cast<uint4*>(sG3 + core_off(128, lt, 8)) = make_uint4(0u, 0u, 0u, 0u);
     }
+    fence_proxy_async();
+    fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      fence_after();
+      // dW3^T[in][out] += H2^T G3 ; dH2 = G3 W3
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        mma(tb + cDW3, mnmaj(sH2, 128, k), mnmaj(sG3, 128, k), kId128x16MM, !(first && k == 0));
+      mma(tb + cZ1, kmaj(sG3, 128, 0), mnmaj(sW3, kOutPad, 0), kId128x128KM, false);
+      commit(bar);
+    }
+    if (!wait_mma()) { failed = true; break; }
+    grad_rows(tb + lrow + cZ1, sS2, lt, c_lo);  // G2
+    fence_proxy_async();
+    fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      fence_after();
+      // dW2[out][in] += G2^T H1 ; db2 += G2^T 1 ; dH1 = G2 W2
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        mma(tb + cDW2, mnmaj(sS2, 128, k), mnmaj(sH1, 128, k), kId128x128MM, !(first && k == 0));
+        mma(tb + cDB2, mnmaj(sS2, 128, k), mnmaj(sOnes, 128, k), kId128x16MM, !(first && k == 0));
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) mma(tb + cZ2, kmaj(sS2, 128, k), mnmaj(sW2, 128, k), kId128x128KM, k > 0);
+      commit(bar);
+    }
+    if (!wait_mma()) { failed = true; break; }
+    grad_rows(tb + lrow + cZ2, sS1, lt, c_lo);  // G1
+    fence_proxy_async();
+    fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      fence_after();
+      // dW1[out][in] += G1^T X ; db1 += G1^T 1
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        mma(tb + cDW1, mnmaj(sS1, 128, k), mnmaj(sX, 128, k), kId128x32MM, !(first && k == 0));
+        mma(tb + cDB1, mnmaj(sS1, 128, k), mnmaj(sOnes, 128, k), kId128x16MM, !(first && k == 0));
+      }
+      commit(bar);
+    }
+    if (!wait_mma()) { failed = true; break; }
+    first = false;
     fence_before();
     __syncthreads();  // TMEM columns and operand buffers free for the next tile
   }
 
-  if (TR && !failed) {
+  if (!failed) {
     float* P = a.partial + (size_t)blockIdx.x * kNPartial;
     if (first) {
-      for (int k = tid; k < kNPartial; k += 128) P[k] = 0.f;
+      for (int k = tid; k < kNPartial; k += kTrainThreads) P[k] = 0.f;
     } else {
+      // a row per lane: 16-byte stores where the caller's rows allow them
+      const bool al = (reinterpret_cast<uintptr_t>(a.partial) & 15u) == 0;
       float v[32];
 #pragma unroll 1
-      for (int c0 = 0; c0 < kHid; c0 += 32) {
+      for (int c0 = c_lo; c0 < c_lo + kHid / 2; c0 += 32) {
         tmem_ld32(tb + lrow + cDW2 + c0, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) P[kOffW2 + tid * kHid + c0 + j] = v[j];
+        store_cols<32>(P + kOffW2 + lt * kHid + c0, v, al);
       }
-      tmem_ld32(tb + lrow + cDW1, v);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) P[kOffW1 + tid * kIn + j] = v[j];
       float u[16];
-      tmem_ld16(tb + lrow + cDW3, u);
+      tmem_ld16(tb + lrow + cDW1 + 16 * half, u);
+      store_cols<16>(P + kOffW1 + lt * kIn + 16 * half, u, al);
+      if (half == 0) {
+        tmem_ld16(tb + lrow + cDW3, u);
 #pragma unroll
-      for (int k = 0; k < kOut; ++k) P[kOffW3 + k * kHid + tid] = u[k];
-      tmem_ld16(tb + lrow + cDB1, u);
-      P[kOffB1 + tid] = u[0];
-      tmem_ld16(tb + lrow + cDB2, u);
-      P[kOffB2 + tid] = u[0];
+        for (int k = 0; k < kOut; ++k) P[kOffW3 + k * kHid + lt] = u[k];
+      } else {
+        tmem_ld16(tb + lrow + cDB1, u);
+        P[kOffB1 + lt] = u[0];
+        tmem_ld16(tb + lrow + cDB2, u);
+        P[kOffB2 + lt] = u[0];
+      }
     }
     // db3 and the loss: warp sums, then warps in order
 #pragma unroll
     for (int k = 0; k < kOut; ++k) r_db3[k] = warp_sum(r_db3[k]);
     r_loss = warp_sum(r_loss);
-    if (lane == 0) {
+    if (lane == 0 && half == 0) {
 #pragma unroll
       for (int k = 0; k < kOut; ++k) s_red[warp * 8 + k] = r_db3[k];
       s_red[warp * 8 + 4] = r_loss;
@@ -434,18 +650,40 @@ __global__ void __launch_bounds__(128, 1) k_mlp(MlpArgs a) {
     mbar_wait(bar, phase);
     __syncthreads();
   }
-  if (warp == 0) tmem_dealloc(tb, L::NCOLS);
+  if (warp == 0) tmem_dealloc(tb, 512);
 }
 
 // Adam (fp32, no weight decay) with a deterministic reduction of the
 // partial rows; every operation rounds separately (no contraction) so a
-// float32 host restatement reproduces it bit for bit.
-__global__ void k_adam(float* w, float* m1, float* m2, const float* partial, int nparts, float lr, float b1, float b2,
-                       float eps, float bc1, float bc2, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3p) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kNParam) return;
+// float32 host restatement reproduces it bit for bit.  The sum over the rows
+// is serial; its loads are not: a CTA copies kAdamRows rows of its kAdamCols
+// parameters into shared memory asynchronously, kAdamLoaders threads to a
+// column, then one thread per column adds them in order.  With a thread
+// loading and adding row after row 148 rows took 6.5 us; this way 5.2 us.
+constexpr int kAdamRows = 152, kAdamCols = 64, kAdamLoaders = 4;
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr(dst)), "l"(src) : "memory");
+}
+__global__ void __launch_bounds__(kAdamCols * kAdamLoaders)
+    k_adam(float* w, float* m1, float* m2, const float* partial, int nparts, float lr, float b1, float b2, float eps,
+           float bc1, float bc2, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3p) {
+  __shared__ float s_p[kAdamRows][kAdamCols];
+  const int col = threadIdx.x % kAdamCols, q = threadIdx.x / kAdamCols;
+  const int k = blockIdx.x * kAdamCols + col;
   float g = 0.f;
-  for (int c = 0; c < nparts; ++c) g = __fadd_rn(g, partial[(size_t)c * kNPartial + k]);
+  for (int c0 = 0; c0 < nparts; c0 += kAdamRows) {
+    const int rows = min(kAdamRows, nparts - c0);
+    if (k < kNParam)
+      for (int r = q; r < rows; r += kAdamLoaders) cp_async4(&s_p[r][col], partial + (size_t)(c0 + r) * kNPartial + k);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (q == 0) {
+#pragma unroll 16
+      for (int r = 0; r < rows; ++r) g = __fadd_rn(g, s_p[r][col]);
+    }
+    __syncthreads();
+  }
+  if (q != 0 || k >= kNParam) return;
   const float m = __fadd_rn(__fmul_rn(b1, m1[k]), __fmul_rn(__fsub_rn(1.0f, b1), g));
   const float v = __fadd_rn(__fmul_rn(b2, m2[k]), __fmul_rn(__fsub_rn(1.0f, b2), __fmul_rn(g, g)));
   m1[k] = m;
@@ -516,9 +754,9 @@ cudaError_t init_mlp_kernels(int* sms) {
   if (!d.done || ctx == 0 || ctx != d.ctx) {
     int n = 0;
     e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (!e) e = cudaFuncSetAttribute(k_mlp<kPredict>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<kPredict>::ALLOC);
-    if (!e) e = cudaFuncSetAttribute(k_mlp<kCorrect>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<kCorrect>::ALLOC);
-    if (!e) e = cudaFuncSetAttribute(k_mlp<kTrain>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<kTrain>::ALLOC);
+    if (!e) e = cudaFuncSetAttribute(k_mlp_infer<kPredict>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlloc);
+    if (!e) e = cudaFuncSetAttribute(k_mlp_infer<kCorrect>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlloc);
+    if (!e) e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlloc);
     if (e) {
       d.done = false;
       return e;
@@ -581,8 +819,8 @@ cudaError_t launch_mlp_correct(const Mlp& m, const KParams& kp, const void* tile
   a.dprev = dprev;
   a.oa = oa;
   a.ob = ob;
-  const int grid = std::min(a.ntiles, 2 * sms);
-  k_mlp<kCorrect><<<grid, 128, Smem<kCorrect>::ALLOC, st>>>(a);
+  const int grid = std::min(a.ntiles, sms);
+  k_mlp_infer<kCorrect><<<grid, 128 * kInferTiles, kAlloc, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -598,8 +836,8 @@ cudaError_t launch_mlp_forward(const Mlp& m, const void* tiles, int n, float* ou
   a.nrows = n;
   a.out = reinterpret_cast<float4*>(out);
   a.flags = flags;
-  const int grid = std::min(a.ntiles, 2 * sms);
-  if (grid > 0) k_mlp<kPredict><<<grid, 128, Smem<kPredict>::ALLOC, st>>>(a);
+  const int grid = std::min(a.ntiles, sms);
+  if (grid > 0) k_mlp_infer<kPredict><<<grid, 128 * kInferTiles, kAlloc, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -619,7 +857,7 @@ cudaError_t launch_mlp_grad(const Mlp& m, const void* tiles, const float* y, con
   a.partial = partial;
   a.flags = flags;
   const int grid = std::max(1, std::min(ntiles, sms));
-  k_mlp<kTrain><<<grid, 128, Smem<kTrain>::ALLOC, st>>>(a);
+  k_mlp_train<<<grid, kTrainThreads, kAlloc, st>>>(a);
   *nparts = grid;
   return cudaGetLastError();
 }
@@ -629,7 +867,7 @@ cudaError_t launch_mlp_adam(Mlp& m, const float* partial, int nparts, float lr, 
   m.step += 1;
   const float bc1 = (float)(1.0 - std::pow((double)b1, (double)m.step));
   const float bc2 = (float)(1.0 - std::pow((double)b2, (double)m.step));
-  k_adam<<<(kNParam + 255) / 256, 256, 0, st>>>(m.w, m.m1, m.m2, partial, nparts, lr, b1, b2, eps, bc1, bc2, bf(m.w1),
+  k_adam<<<(kNParam + kAdamCols - 1) / kAdamCols, kAdamCols * kAdamLoaders, 0, st>>>(m.w, m.m1, m.m2, partial, nparts, lr, b1, b2, eps, bc1, bc2, bf(m.w1),
                                                 bf(m.w2), bf(m.w3p));
   return cudaGetLastError();
 }
