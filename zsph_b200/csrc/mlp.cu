@@ -777,6 +777,47 @@ int fail_cuda(cudaError_t e, const char* what) {
   return fail(ZSPH_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+// A status word for one call of a network's entry points: the kernels OR
+// ZSPH_FLAG_TIMEOUT into it, the host reads it after the stream's
+// synchronisation.  The words are pinned host memory the GPU writes directly
+// (only when a wait times out), kFlagWords of them per network, 64 bytes
+// apart, handed out under a lock so that concurrent calls on one network stay
+// apart; a call that finds none free gets memory of its own.  A cudaMalloc,
+// a clear, a copy back and a cudaFree per call took 25-30 us.
+class CallFlag {
+ public:
+  explicit CallFlag(Mlp& m) : m_(m) {
+    {
+      std::lock_guard<std::mutex> lk(m_.flag_mu);
+      for (int k = 0; k < kFlagWords && idx_ < 0; ++k)
+        if (!(m_.flag_used >> k & 1u)) idx_ = k;
+      if (idx_ >= 0) m_.flag_used |= 1u << idx_;
+    }
+    if (idx_ >= 0) word_ = m_.flag_words + 16 * idx_;
+    else if ((err_ = cudaHostAlloc(&word_, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable))) word_ = nullptr;
+    if (word_) *word_ = 0;
+  }
+  ~CallFlag() {
+    if (idx_ >= 0) {
+      std::lock_guard<std::mutex> lk(m_.flag_mu);
+      m_.flag_used &= ~(1u << idx_);
+    } else if (word_) {
+      cudaFreeHost(word_);
+    }
+  }
+  CallFlag(const CallFlag&) = delete;
+  CallFlag& operator=(const CallFlag&) = delete;
+  cudaError_t error() const { return err_; }
+  int* device() const { return word_; }  // one address on both sides (unified addressing)
+  int read() const { return *static_cast<volatile int*>(word_); }
+
+ private:
+  Mlp& m_;
+  int idx_ = -1;
+  int* word_ = nullptr;
+  cudaError_t err_ = cudaSuccess;
+};
+
 // splitmix64
 uint64_t mix64(uint64_t& s) {
   uint64_t z = (s += 0x9E3779B97F4A7C15ull);
@@ -898,8 +939,10 @@ int zsph_mlp_create(unsigned long long seed, zsph_mlp_t** out) {
   auto* m = new zsph_mlp();
   cudaError_t e = cudaMalloc(&m->w, sizeof(float) * kNParam * 3);
   if (!e) e = cudaMalloc(&m->w1, sizeof(__nv_bfloat16) * (kHid * kIn + kHid * kHid + kOutPad * kHid));
+  if (!e) e = cudaHostAlloc(&m->flag_words, 64 * kFlagWords, cudaHostAllocMapped | cudaHostAllocPortable);
   if (e) {
     cudaFree(m->w);
+    cudaFree(m->w1);
     delete m;
     return fail(ZSPH_ENOMEM, std::string("zsph_mlp_create: ") + cudaGetErrorString(e));
   }
@@ -940,6 +983,7 @@ int zsph_mlp_destroy(zsph_mlp_t* m) {
   if (!m) return ZSPH_OK;
   cudaFree(m->w);
   cudaFree(m->w1);
+  cudaFreeHost(m->flag_words);
   delete m;
   return ZSPH_OK;
 }
@@ -1008,16 +1052,12 @@ int zsph_mlp_forward(zsph_mlp_t* m, const void* tiles, int n, float* out, void* 
   if (!m || n < 0 || (n > 0 && (!tiles || !out))) return fail(ZSPH_EINVAL, "zsph_mlp_forward: bad argument");
   if ((reinterpret_cast<uintptr_t>(tiles) | reinterpret_cast<uintptr_t>(out)) & 15)
     return fail(ZSPH_EINVAL, "zsph_mlp_forward: tiles and out must be 16-byte aligned");
-  int* flags = nullptr;
-  cudaError_t e = cudaMalloc(&flags, sizeof(int));
-  if (!e) e = cudaMemset(flags, 0, sizeof(int));
-  if (!e) e = launch_mlp_forward(*m, tiles, n, out, flags, static_cast<cudaStream_t>(stream));
-  int f = 0;
-  if (!e) e = cudaMemcpyAsync(&f, flags, sizeof(int), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
+  const CallFlag flag(*m);
+  cudaError_t e = flag.error();
+  if (!e) e = launch_mlp_forward(*m, tiles, n, out, flag.device(), static_cast<cudaStream_t>(stream));
   if (!e) e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-  cudaFree(flags);
   if (e) return fail_cuda(e, "zsph_mlp_forward");
-  return (f & ZSPH_FLAG_TIMEOUT) ? fail(ZSPH_ETIMEOUT, "zsph_mlp_forward: tensor-core wait timed out") : ZSPH_OK;
+  return (flag.read() & ZSPH_FLAG_TIMEOUT) ? fail(ZSPH_ETIMEOUT, "zsph_mlp_forward: tensor-core wait timed out") : ZSPH_OK;
 }
 
 int zsph_mlp_grad(zsph_mlp_t* m, const void* tiles, const float* y, const float* w, const int* tile_ids, int ntiles,
@@ -1026,18 +1066,14 @@ int zsph_mlp_grad(zsph_mlp_t* m, const void* tiles, const float* y, const float*
     return fail(ZSPH_EINVAL, "zsph_mlp_grad: bad argument");
   if ((reinterpret_cast<uintptr_t>(tiles) | reinterpret_cast<uintptr_t>(y)) & 15)
     return fail(ZSPH_EINVAL, "zsph_mlp_grad: tiles and y must be 16-byte aligned");
-  int* flags = nullptr;
-  cudaError_t e = cudaMalloc(&flags, sizeof(int));
-  if (!e) e = cudaMemset(flags, 0, sizeof(int));
+  const CallFlag flag(*m);
+  cudaError_t e = flag.error();
   if (!e)
-    e = launch_mlp_grad(*m, tiles, y, w, tile_ids, ntiles, inv_wsum, partial, nparts, flags,
+    e = launch_mlp_grad(*m, tiles, y, w, tile_ids, ntiles, inv_wsum, partial, nparts, flag.device(),
                         static_cast<cudaStream_t>(stream));
-  int f = 0;
-  if (!e) e = cudaMemcpyAsync(&f, flags, sizeof(int), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
   if (!e) e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-  cudaFree(flags);
   if (e) return fail_cuda(e, "zsph_mlp_grad");
-  return (f & ZSPH_FLAG_TIMEOUT) ? fail(ZSPH_ETIMEOUT, "zsph_mlp_grad: tensor-core wait timed out") : ZSPH_OK;
+  return (flag.read() & ZSPH_FLAG_TIMEOUT) ? fail(ZSPH_ETIMEOUT, "zsph_mlp_grad: tensor-core wait timed out") : ZSPH_OK;
 }
 
 int zsph_mlp_adam(zsph_mlp_t* m, const float* partial, int nparts, float lr, float beta1, float beta2, float eps,

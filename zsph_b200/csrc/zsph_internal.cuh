@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "../../include/zsph.h"
@@ -354,7 +355,12 @@ struct Mlp {
   // input / output standardization of the learned corrector
   float in_mean[kFeat], in_inv_std[kFeat];
   float out_mean[4], out_std[4];
+  // status words of the calls in flight (mlp.cu, CallFlag): pinned host memory, 64 bytes each
+  int* flag_words = nullptr;
+  unsigned flag_used = 0;
+  std::mutex flag_mu;
 };
+constexpr int kFlagWords = 32;
 cudaError_t launch_mlp_correct(const Mlp& m, const KParams& kp, const void* tiles, const zsph_ptc_t& ptc,
                                float4* acc, const float4* dprev, float4 oa, float4 ob, int* flags, cudaStream_t st);
 cudaError_t launch_mlp_forward(const Mlp& m, const void* tiles, int n, float* out, int* flags, cudaStream_t st);
