@@ -57,3 +57,25 @@ def test_walls_with_overflowed_lists():
     for a in range(2):
         assert np.abs(new[:, a] - want[:, a]).max() <= 1e-4 * max(np.abs(want[:, a]).max(), 1e-30)
     sol.close()
+
+
+@pytest.mark.parametrize("n,box", [(4001, (0.4, 0.3, 0.3)), (31, (0.2, 0.2, 0.2)), (64013, (1.5, 1.0, 0.6))])
+def test_lists_of_crowded_and_empty_rows(n, box):
+    """Neighbour counts of a list build with rows of no candidates, of more
+    than 64, lists past their capacity and a particle at NaN, in both forms of
+    the build, against the oracle (exact; -1 marks an overflowed list)."""
+    c = cases.random_cloud(n, 9, box=box)
+    mid, k = c.state.pos.mean(0), n // 8
+    c.state.pos[:k] = mid + (c.state.pos[:k] - mid) * 0.25
+    c.state.pos[n // 2] = np.nan
+    c.state.tmp_pos[:] = c.state.pos
+    sol = z.Solver.from_case(c)
+    sol.neighbor_search("old", "new")
+    nb_b, nb_g = sol.neighbor_counts("new")
+    o = po.Oracle(c.json, c.state, np.float32)
+    o.search()
+    for got, want in ((nb_b, o.neighbor_count("new", "boundary")), (nb_g, o.neighbor_count("new", "governing"))):
+        full = o.neighbor_count("new", "governing") > 128
+        assert full.any() or n < 100
+        assert np.array_equal(got, np.where(full, -1, want))
+    sol.close()

@@ -450,12 +450,18 @@ constexpr int kCellWarps = 4;  // warps per CTA in the list build
 // Testing the union of the segments' ranges instead (one set of arrays)
 // costs 1.6x the candidate tests on the dam-break cases.  Hits come out in
 // candidate order, so a list is in the reference's visit order, and its
-// entries are offsets from the lane's row start.  Each lane emits the hits
-// of a 16-candidate half block into its 32-entry ring in shared memory;
-// after the half, the lanes write their completed 8-entry blocks together (a
-// nearly converged loop) with 16-byte stores to the blocked list layout.
-// Flushing at a lane's 8th entry inside the per-hit loop instead diverges:
-// each flush then runs for 2-3 lanes.
+// entries are offsets from the lane's row start.
+//
+// Emission.  The tests leave one 32-bit word of hits per 32 candidates; a
+// lane queues its words that are not empty, and when a queue is full, and at
+// the end, the lanes emit their entries together, eight per iteration, packed
+// in registers and stored as one 16-byte block.  All lanes have entries left
+// in nearly every iteration, whatever row they come from: the iterations are
+// the longest list's, about 10 blocks.  Emitting each half word of 16
+// candidates as it was tested (a loop as long as the fullest lane's hits in
+// it, into a ring) cost 2.5 times the iterations: 1446 against 1220 us at
+// 4.2 M particles, 62.7 against 54.5 at 105 k; with queues of 8 words instead
+// of 16 (less shared memory, more drains) 1251 and 57.2.
 //
 // Precision form: candidates are moved into the frame of the lane's own
 // cell (its position is the offset from that cell's corner, as in the pair
@@ -463,11 +469,54 @@ constexpr int kCellWarps = 4;  // warps per CTA in the list build
 // is exact and one rounding forms every coordinate.
 //
 // The walls' (rho, p) come after, from the finished lists (k_walls).
-constexpr int kRing = 32;  // list-build ring entries per lane (power of two)
+// list build: hit words queued per lane (a power of two, more than 7; less with many warps' shared memory)
+template <int CW> constexpr int kQueueOf = CW > 4 ? 8 : 16;
 constexpr int kSegs = 4;   // list build: cells whose lanes test their own rows concurrently
 constexpr int kStage = 66; // list build: staged candidates per segment (64) plus two floats of padding
 // warps per CTA of k_nblist_seq (the 5x5 stencil's row starts need more shared memory)
 template <int GF> constexpr int kSeqWarps = GF == 1 ? kCellWarps : 2;
+
+// Neighbour tests of one lane's position (each coordinate twice) against 32
+// staged candidates (x at sx, y and z at kStage, 2 * kStage), two per step
+// with packed arithmetic; only the first `left` are candidates, the blocks of
+// eight beyond are skipped.  Bit 31 - k: candidate k within r2max (mh), and
+// with SKIN within r2skin (mk).  A hit's bit is the sign of r^2 less the next
+// float above the threshold (exact in sign; a NaN of the operation is
+// positive, no hit), shifted in: one packed subtraction and a shift per
+// candidate instead of a compare and a predicated OR, 1196 against 1220 us at
+// 4.2 M particles.
+template <bool SKIN>
+__device__ __forceinline__ void hits32(const float* sx, u64 px, u64 py, u64 pz, float r2max, float r2skin, int left,
+                                       unsigned& mh, unsigned& mk) {
+  // r^2 <= r2max <=> r^2 - (the next float above r2max) < 0
+  const float lim = __uint_as_float(__float_as_uint(r2max) + 1u), lims = __uint_as_float(__float_as_uint(r2skin) + 1u);
+  const u64 lim2 = pk2(lim, lim), lims2 = pk2(lims, lims);
+  int n = 0;
+#pragma unroll
+  for (int blk = 0; blk < 4; ++blk) {
+    if (8 * blk >= left) break;  // uniform: the rest is padding
+    n += 8;
+#pragma unroll
+    for (int tt = 8 * blk; tt < 8 * blk + 8; tt += 2) {
+      const u64 x2 = *reinterpret_cast<const u64*>(&sx[tt]);
+      const u64 y2 = *reinterpret_cast<const u64*>(&sx[kStage + tt]);
+      const u64 z2 = *reinterpret_cast<const u64*>(&sx[2 * kStage + tt]);
+      const u64 dx = sub2(px, x2), dy = sub2(py, y2), dz = sub2(pz, z2);
+      const u64 d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+      float r0, r1;
+      upk2(sub2(d2, lim2), r0, r1);
+      mh = __funnelshift_l(__float_as_uint(r0), mh, 1);
+      mh = __funnelshift_l(__float_as_uint(r1), mh, 1);
+      if constexpr (SKIN) {
+        upk2(sub2(d2, lims2), r0, r1);
+        mk = __funnelshift_l(__float_as_uint(r0), mk, 1);
+        mk = __funnelshift_l(__float_as_uint(r1), mk, 1);
+      }
+    }
+  }
+  mh <<= (32 - n) & 31;
+  if constexpr (SKIN) mk <<= (32 - n) & 31;
+}
 
 // At least 42 warps per SM (a register budget of 40-48 without spills in the
 // plain form, 9.9 KB of shared memory per 2-warp CTA): the kernel is
@@ -484,9 +533,8 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
   // per segment (cell) of a round: its 64 staged candidates' x, y and z; the
   // two floats of padding per array put the segments' arrays in different banks
   __shared__ __align__(16) float s_c[CW][SEGS][3][kStage];
-  // per lane: a 32-entry ring (a partial 8-entry block plus one half block's
-  // hits fit), padded to 80 bytes so that the lanes' rings spread over the banks
-  __shared__ __align__(16) uint16_t s_ring[CW][32][kRing + 8];
+  constexpr int kQueue = kQueueOf<CW>;
+  __shared__ uint2 s_q[CW][kQueue][32];  // per lane: the queue of hit words
   const int lane = threadIdx.x & 31;
   const int p0 = group * 32;
   if (p0 >= kp_arg.n) return;  // uniform per warp
@@ -506,21 +554,45 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
   const KParams kp = BATCH ? scene_kp(kp_arg, scn) : kp_arg;
   const float r2max = kp.r2max;
   const u64 px = pk2(pi.x, pi.x), py = pk2(pi.y, pi.y), pz = pk2(pi.z, pi.z);
-  uint16_t* ring = s_ring[wid][lane];
   uint4* nbv = reinterpret_cast<uint4*>(s.nb);
-  int cnt = 0;   // entries emitted
+  int cnt = 0;   // hits found
   int done = 0;  // entries written to global memory (a multiple of 8)
   bool ovf = false;
+  // the lane's queue of hit words (first bit = first candidate) and the entry
+  // of each word's first candidate; cur / cent: the word being emitted
+  int qh = 0, qn = 0;
+  unsigned cur = 0u, cent = 0u;
   // SKIN (the list transfer's predictor): the candidates with
   // r2max < r^2 <= r2skin, in candidate order, into the skin list
   const float r2skin = kp.r2skin;
   int kc = 0;
   bool skovf = false;
-  // writes the completed 8-entry blocks among the first min(cnt, kMaxNb) entries
-  auto flush = [&]() {
-    const int lim = min(cnt, kMaxNb);
-    for (; done + 8 <= lim; done += 8)
-      nbv[nb_vec(i, done >> 3)] = *reinterpret_cast<const uint4*>(ring + (done & (kRing - 1)));
+  // emits the queued hits eight at a time; `all`: the last, partial block too
+  auto drain = [&](bool all) {
+    for (;;) {
+      const bool more = !ovf && (all ? done < cnt : done + 8 <= cnt);
+      if (!__any_sync(0xffffffffu, more)) break;
+      if (more) {
+        unsigned w[4];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          if (cur == 0u) {  // past the last hit: any slot, the entry is never read
+            const uint2 v = s_q[wid][qh][lane];
+            cur = v.x;
+            cent = v.y;
+            qh = (qh + 1) % kQueue;
+            --qn;
+          }
+          const int bb = __clz(cur);
+          cur &= ~(0x80000000u >> (bb & 31));
+          const unsigned ent = cent + (unsigned)bb;
+          if (e & 1) w[e >> 1] |= ent << 16;
+          else w[e >> 1] = ent & 0xffffu;
+        }
+        nbv[nb_vec(i, done >> 3)] = make_uint4(w[0], w[1], w[2], w[3]);
+        done += 8;
+      }
+    }
   };
   // The lanes of one cell are contiguous (sorted particles).  A round takes
   // the next kSegs cells (segments): per stencil row each segment's range is
@@ -569,37 +641,18 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
           const int base = k0 + 32 * h;  // offset of the block in the lane's row range
           if (base >= L) break;          // uniform
           unsigned mh = 0u, mk = 0u;
-#pragma unroll
-          for (int blk = 0; blk < 4; ++blk) {
-            if (base + 8 * blk >= L) break;  // uniform: the rest is padding
-#pragma unroll
-            for (int tt = 8 * blk; tt < 8 * blk + 8; tt += 2) {
-              const u64 x2 = *reinterpret_cast<const u64*>(&sx[32 * h + tt]);
-              const u64 y2 = *reinterpret_cast<const u64*>(&sx[kStage + 32 * h + tt]);
-              const u64 z2 = *reinterpret_cast<const u64*>(&sx[2 * kStage + 32 * h + tt]);
-              const u64 dx = sub2(px, x2), dy = sub2(py, y2), dz = sub2(pz, z2);
-              const u64 d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-              float r0, r1;
-              upk2(d2, r0, r1);
-              if (r0 <= r2max) mh |= 1u << tt;
-              if (r1 <= r2max) mh |= 2u << tt;
-              if constexpr (SKIN) {
-                if (r0 <= r2skin) mk |= 1u << tt;
-                if (r1 <= r2skin) mk |= 2u << tt;
-              }
-            }
-          }
+          hits32<SKIN>(sx + 32 * h, px, py, pz, r2max, r2skin, L - base, mh, mk);
           // keep the hits inside this lane's range (offsets < len), not itself
           const int hi = len - base;
-          unsigned keep = hi <= 0 ? 0u : (hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u));
+          unsigned keep = hi <= 0 ? 0u : (hi >= 32 ? 0xffffffffu : ~(0xffffffffu >> hi));
           const int self = i - sl - base;
-          if (self >= 0 && self < 32) keep &= ~(1u << self);
+          if (self >= 0 && self < 32) keep &= ~(0x80000000u >> self);
           mh &= keep;
           if constexpr (SKIN) {
             mk &= keep & ~mh;
             while (mk) {
-              const int bb = __ffs(mk) - 1;
-              mk &= mk - 1;
+              const int bb = __clz(mk);
+              mk &= ~(0x80000000u >> bb);
               const int off = base + bb;
               if (kc < kSkinCap && off <= kOffMask)
                 s.xf.sk[sk_idx(i, kc)] = (uint16_t)(((unsigned)r << kRowShift) | (unsigned)off);
@@ -608,44 +661,26 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
               ++kc;
             }
           }
-          if (!mh) continue;
-          const int off0 = base;
-          if (cnt + __popc(mh) <= kMaxNb && off0 + 31 <= kOffMask) {
-#pragma unroll
-            for (int hb = 0; hb < 32; hb += 16) {  // one half block, then its flush
-              const unsigned ent0 = ((unsigned)r << kRowShift) + (unsigned)(off0 + hb);
-              unsigned part = (mh >> hb) & 0xffffu;
-              while (part) {
-                const int bb = __ffs(part) - 1;
-                part &= part - 1;
-                ring[cnt & (kRing - 1)] = (uint16_t)(ent0 + bb);
-                ++cnt;
-              }
-              flush();
-            }
-          } else {
-#pragma unroll
-            for (int hb = 0; hb < 32; hb += 16) {
-              unsigned part = (mh >> hb) & 0xffffu;
-              while (part) {
-                const int bb = __ffs(part) - 1;
-                part &= part - 1;
-                const int off = off0 + hb + bb;
-                if (cnt < kMaxNb && off <= kOffMask && !ovf)
-                  ring[cnt & (kRing - 1)] = (uint16_t)(((unsigned)r << kRowShift) | (unsigned)off);
-                else
-                  ovf = true;
-                ++cnt;
-              }
-              flush();
+          if (base + 31 > kOffMask && mh != 0u) {  // offsets a list entry cannot hold
+            const int fit = kOffMask + 1 - base;   // candidates of the word it can
+            if (fit <= 0 || (mh & (0xffffffffu >> fit)) != 0u) ovf = true;
+          }
+          if (mh != 0u) {
+            cnt += __popc(mh);
+            if (cnt > kMaxNb) ovf = true;
+            if (ovf) {
+              qn = 0;
+            } else {
+              s_q[wid][(qh + qn) % kQueue][lane] = make_uint2(mh, ((unsigned)r << kRowShift) + (unsigned)base);
+              ++qn;
             }
           }
+          if (__any_sync(0xffffffffu, qn == kQueue)) drain(false);
         }
       }
     }
   }
-  if (cnt > 254) ovf = true;
-  if (act && !ovf && (cnt & 7)) nbv[nb_vec(i, cnt >> 3)] = *reinterpret_cast<const uint4*>(ring + (cnt & (kRing - 8)));
+  drain(true);
   if (SKIN && act) s.xf.sk_cnt[i] = skovf ? kOverflow : (uint8_t)kc;
   if (act) {
     const bool fluid_nb = GF != 1 || fluid_of(pi.w) || walls_fluid_near(kp, s, t, c);
@@ -1461,7 +1496,8 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
     if (GF != 1) return cudaErrorInvalidValue;
     k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
   } else {
-    k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
+    if (GF == 1) launch_nblist_tuned<false>(kp, s, ptc, t, st);
+    else k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
   }
   return cudaGetLastError();
 }
