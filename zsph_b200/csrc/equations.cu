@@ -696,6 +696,137 @@ __global__ void __launch_bounds__(CW * 32, 42 / CW) k_nblist_seq(KParams kp_arg,
   nblist_group<GF, CW, BATCH, PRECISE, SEGS, SKIN>(kp_arg, s, ptc, t, blockIdx.x * CW + wid, wid);
 }
 
+// The list build of a small case: a CTA of three warps per 32 particles, one
+// warp per z-plane of the 3x3 stencil rows, so that a group's serial chain
+// (row bounds, staging, tests, emission, row after row) is a third as long.
+// Each warp collects its plane's entries per lane in shared memory; the
+// planes' entries in order are the list, so it equals k_nblist_seq's entry
+// for entry.  13 k / 20 k / 34 k / 54 k particles: 21 / 24 / 31 / 36 us, against
+// 35 / 37 / 43 / 44 with one warp per group; equal at 61 k, and slower from
+// 105 k on (68 against 53), where warps are plenty and the planes' buffers
+// limit how many are resident.
+constexpr int kPlanes = 3;
+constexpr int kPlaneCap = kMaxNb + 2;  // 65 words per lane: the lanes' k-th entries fall in different banks
+constexpr int kSplitMax = 56000;
+
+template <bool BATCH, bool PRECISE>
+__global__ void __launch_bounds__(32 * kPlanes) k_nblist_split(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
+                                                               zsph_tmp_t t) {
+  constexpr int GF = 1, SEGS = kSegs;
+  __shared__ __align__(16) float s_c[kPlanes][SEGS][3][kStage];
+  __shared__ uint16_t s_e[kPlanes][32][kPlaneCap];
+  __shared__ int s_n[kPlanes][32];  // entries found (kMaxNb + 1: one could not be stored)
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int p0 = blockIdx.x * 32;
+  const int i = p0 + lane;
+  const bool act = i < kp_arg.n;
+  const int c = act ? t.hash[i] : INT_MAX;  // sorted: non-decreasing over the lanes
+  const int scn = BATCH && act ? scene_of(kp_arg.scene_cbase, kp_arg.nscenes, c) : 0;
+  const KParams kp = BATCH ? scene_kp(kp_arg, scn) : kp_arg;
+  const int iself = act ? i : p0;
+  const float2 rp_self = reinterpret_cast<const float2*>(ptc.rhop)[iself];
+  const float4 pi = make_float4(ptc.pos[3 * iself], ptc.pos[3 * iself + 1], ptc.pos[3 * iself + 2],
+                                packed_rho(rp_self.x, ptc.type[iself]));
+  const int3 ci = PRECISE && act ? unpack_cell(kp_arg.c3n[i]) : int3{0, 0, 0};
+  const u64 px = pk2(pi.x, pi.x), py = pk2(pi.y, pi.y), pz = pk2(pi.z, pi.z);
+  uint16_t* buf = s_e[wid][lane];
+  int cnt = 0;
+  bool ovf = false;
+  int rs[3], rl[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    int e = 0;
+    rs[k] = 0;
+    if (act) row_range<GF>(kp, t, c, 3 * wid + k, rs[k], e);
+    rl[k] = act ? max(e - rs[k], 0) : 0;
+  }
+  const int cprev = __shfl_up_sync(0xffffffffu, c, 1);
+  const unsigned starts = __ballot_sync(0xffffffffu, act && (lane == 0 || c != cprev));
+  unsigned todo = __ballot_sync(0xffffffffu, act);
+  while (todo) {  // rounds of up to SEGS cells, as in nblist_group
+    const unsigned sm = starts & todo;
+    const int seg = ((todo >> lane) & 1u) ? __popc(sm & (0xffffffffu >> (31 - lane))) - 1 : SEGS;
+    const bool inseg = seg < SEGS;
+    todo &= ~__ballot_sync(0xffffffffu, inseg);
+    const int nseg = min(__popc(sm), SEGS);
+    const float* sx = s_c[wid][inseg ? seg : 0][0];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int sl = rs[k], len = inseg ? rl[k] : 0;
+      const int L = __reduce_max_sync(0xffffffffu, len);
+      for (int k0 = 0; k0 < L; k0 += 64) {
+        __syncwarp();
+        unsigned m = sm;
+        for (int g = 0; g < nseg; ++g) {  // uniform
+          const int lead = __ffs(m) - 1;
+          m &= m - 1;
+          const int sg = __shfl_sync(0xffffffffu, sl, lead), lg = __shfl_sync(0xffffffffu, len, lead);
+          int3 cg{0, 0, 0};
+          if (PRECISE)
+            cg = make_int3(__shfl_sync(0xffffffffu, ci.x, lead), __shfl_sync(0xffffffffu, ci.y, lead),
+                           __shfl_sync(0xffffffffu, ci.z, lead));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int o = k0 + 32 * h + lane;
+            float4 q = make_float4(3e37f, 3e37f, 3e37f, 0.f);  // padding never passes the test
+            if (o < lg) q = ptc_xyz<PRECISE>(kp, ptc, sg + o, cg);
+            s_c[wid][g][0][32 * h + lane] = q.x;
+            s_c[wid][g][1][32 * h + lane] = q.y;
+            s_c[wid][g][2][32 * h + lane] = q.z;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int base = k0 + 32 * h;
+          if (base >= L) break;  // uniform
+          unsigned mh = 0u, mk = 0u;
+          hits32<false>(sx + 32 * h, px, py, pz, kp.r2max, 0.0f, L - base, mh, mk);
+          const int hi = len - base;  // inside the lane's range, not itself
+          mh &= hi <= 0 ? 0u : (hi >= 32 ? 0xffffffffu : ~(0xffffffffu >> hi));
+          const int self = i - sl - base;
+          if (self >= 0 && self < 32) mh &= ~(0x80000000u >> self);
+          const unsigned ent0 = ((unsigned)(3 * wid + k) << kRowShift) + (unsigned)base;
+          if (cnt + __popc(mh) > kMaxNb || base + 31 > kOffMask) {
+            ovf |= mh != 0u;
+            cnt += __popc(mh);
+            mh = 0u;
+          }
+          while (mh) {
+            const int bb = __clz(mh);
+            mh &= ~(0x80000000u >> bb);
+            buf[cnt++] = (uint16_t)(ent0 + bb);
+          }
+        }
+      }
+    }
+  }
+  s_n[wid][lane] = ovf ? kMaxNb + 1 : cnt;
+  __syncthreads();
+  const int n0 = s_n[0][lane], n1 = s_n[1][lane], n2 = s_n[2][lane];
+  const int tot = n0 + n1 + n2;
+  const bool bad = tot > kMaxNb;
+  if (act && !bad) {
+    uint4* nbv = reinterpret_cast<uint4*>(s.nb);
+    for (int b = wid; 8 * b < tot; b += kPlanes) {
+      unsigned w[4];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int k = 8 * b + e, k1 = k - n0, k2 = k1 - n1;
+        const uint16_t* src = k1 < 0 ? &s_e[0][lane][k] : k2 < 0 ? &s_e[1][lane][k1] : &s_e[2][lane][min(k2, kPlaneCap - 1)];
+        const unsigned v = *src;
+        if (e & 1) w[e >> 1] |= v << 16;
+        else w[e >> 1] = v;
+      }
+      nbv[nb_vec(i, b)] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+  if (wid == 0 && act) {
+    const bool fluid_nb = fluid_of(pi.w) || walls_fluid_near(kp, s, t, c);
+    list_tail<GF, PRECISE>(kp, s, ptc, i, bad ? 0 : tot, bad, pi, rp_self, fluid_nb);
+  }
+}
+
 // The list transfer's fallback: the full list build of the corrector, run
 // only when the transfer's conditions failed this step (*s.xf.flag set);
 // otherwise every CTA returns at once.
@@ -1324,10 +1455,15 @@ __global__ void __launch_bounds__(kSearchBlock) k_integrate(KParams kp, zsph_ptc
 
 inline int thread_blocks(int n) { return (n + kPairBlock - 1) / kPairBlock; }
 
-// list build (grid factor 1) with the tuned number of cells per CTA
+// list build (grid factor 1): a plane per warp for small cases, else with the
+// tuned number of cells per CTA
 template <bool BATCH>
 void launch_nblist_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc, const zsph_tmp_t& t,
                          cudaStream_t st) {
+  if (kp.n <= kSplitMax) {
+    k_nblist_split<BATCH, false><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
+    return;
+  }
   // (eight cells per CTA would exceed the 48 KB of static shared memory)
   // default (0): two warps per CTA, what zsph_autotune picks on the dam-break cases
   // default segments per round (0): four
@@ -1399,7 +1535,8 @@ cudaError_t boundary_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& p
   }
   if (kp.c3o) {  // precision form (grid factor 1, delta equations)
     if (GF != 1 || kp.equations != ZSPH_EQ_DELTA) return cudaErrorInvalidValue;
-    k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
+    if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
+    else k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
     mark(pf, "nblist", st);
     launch_walls<1, true>(kp, s, t, st);
     mark(pf, "walls", st);
@@ -1494,7 +1631,8 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
     launch_nblist_tuned<true>(kp, s, ptc, t, st);
   } else if (kp.c3o) {
     if (GF != 1) return cudaErrorInvalidValue;
-    k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
+    if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
+    else k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
   } else {
     if (GF == 1) launch_nblist_tuned<false>(kp, s, ptc, t, st);
     else k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
