@@ -1198,8 +1198,12 @@ struct FeatAcc {
 // so neighbours still read the unintegrated state).  FEAT (predictor stage
 // of the learned form) also accumulates and writes the FeatOut aggregates.
 // PRECISE: precision form (cell + offset positions).
-// MINB: minimum resident CTAs per SM (register budget); the default six
-// give 80 registers without spills for the plain variants.
+// MINB: minimum resident CTAs per SM (register budget).  The default leaves
+// the registers to the compiler (93 for the plain variants, 110 in the
+// precision form): six CTAs per SM (80 registers, a few spilled in the
+// precision form) took 180 against 155 us with a floating body at 362 k
+// particles and 177 against 163 at 445 k in the drop-in call.  governing_minb
+// has the exception.
 // REUSE: as k_boundary's (entries re-tested at the current positions).
 // governing_one: one thread's particle i, as boundary_one.
 // List transfer, in the predictor's fused integration: particle i's
@@ -1360,7 +1364,7 @@ __device__ __forceinline__ void governing_one(const KParams& kp_arg, const Scrat
 }
 
 template <int GF, int MODE, bool FEAT = false, bool PRECISE = false, bool BATCH = false, bool RIGID = false,
-          int MINB = (FEAT || BATCH) ? 1 : 6, bool REUSE = false>
+          int MINB = 1, bool REUSE = false>
 __global__ void __launch_bounds__(kPairBlock, MINB)
     k_governing(KParams kp_arg, Scratch s, zsph_ptc_t ptc, zsph_tmp_t t, zsph_ptc_t out, FeatOut fo) {
   extern __shared__ __align__(16) unsigned char dsm[];
@@ -1491,16 +1495,33 @@ void launch_nblist_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
   }
 }
 
-// governing (grid factor 1, fused prediction / correction, no shared-memory
-// windows) with the tuned register budget
+inline int sm_count() {
+  static int sms = 0;  // SMs of the device (the same for every B200)
+  if (!sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 148;
+  }
+  return sms;
+}
+
+// Register budget of the plain governing pass when none was tuned: at 93
+// registers five CTAs fit an SM, at 80 six.  A case whose CTAs fit the device
+// at once with six but leave a nearly empty second wave with five (94,720 to
+// 113,664 particles on 148 SMs) takes six: 48.8 against 53.5 us at 105 k.
+inline int governing_minb(int n) {
+  const int ctas = thread_blocks(n), sms = sm_count();
+  return ctas > 5 * sms && ctas <= 6 * sms ? 6 : 1;
+}
+
+// governing (grid factor 1, no shared-memory windows) with the tuned register
+// budget
 template <int MODE, bool BATCH>
 void launch_governing_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc, const zsph_tmp_t& t,
                             const zsph_ptc_t& out, cudaStream_t st) {
   const FeatOut none{};
   const int nb = thread_blocks(kp.n), sm = pair_smem<1>(0, 0);
-  // default (0): one resident CTA minimum (the largest register budget), what
-  // zsph_autotune picks on the dam-break cases
-  switch (kp.tune_minb) {
+  switch (kp.tune_minb ? kp.tune_minb : BATCH ? 1 : governing_minb(kp.n)) {
     case 6: k_governing<1, MODE, false, false, BATCH, false, 6><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
     case 8: k_governing<1, MODE, false, false, BATCH, false, 8><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
     default: k_governing<1, MODE, false, false, BATCH, false, 1><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
@@ -1510,14 +1531,8 @@ void launch_governing_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_
 // CTAs of a wall pass with `lanes` lanes per wall: enough to fill the device,
 // each looping over s.wl (its length is known on the device only).
 inline int walls_grid(int n, int lanes) {
-  static int sms = 0;  // SMs of the device (the same for every B200)
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 148;
-  }
   const int per_cta = kPairBlock / lanes;
-  return min((n + per_cta - 1) / per_cta, sms * 16);
+  return min((n + per_cta - 1) / per_cta, sm_count() * 16);
 }
 template <int GF, bool PRECISE = false, bool BATCH = false>
 void launch_walls(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, cudaStream_t st) {
@@ -1547,7 +1562,7 @@ cudaError_t boundary_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& p
   if (kp.c3o) {  // precision form (grid factor 1, delta equations)
     if (GF != 1 || kp.equations != ZSPH_EQ_DELTA) return cudaErrorInvalidValue;
     if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
+    else k_nblist_seq<1, 2, false, true><<<(kp.n + 63) / 64, 64, 0, st>>>(kp, s, ptc, t);
     mark(pf, "nblist", st);
     launch_walls<1, true>(kp, s, t, st);
     mark(pf, "walls", st);
@@ -1621,7 +1636,8 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     mark(pf, "governing", st);
     return cudaGetLastError();
   }
-  if (GF == 1 && !kp.stage_windows && mode != 0) {
+  if (GF == 1 && !kp.stage_windows) {
+    if (mode == 0) launch_governing_tuned<0, false>(kp, s, ptc, t, out, st);
     if (mode == 1) launch_governing_tuned<1, false>(kp, s, ptc, t, out, st);
     if (mode == 2) launch_governing_tuned<2, false>(kp, s, ptc, t, out, st);
     mark(pf, "governing", st);
@@ -1643,7 +1659,7 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
   } else if (kp.c3o) {
     if (GF != 1) return cudaErrorInvalidValue;
     if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, kCellWarps, false, true><<<(kp.n + 32 * kCellWarps - 1) / (32 * kCellWarps), kCellWarps * 32, 0, st>>>(kp, s, ptc, t);
+    else k_nblist_seq<1, 2, false, true><<<(kp.n + 63) / 64, 64, 0, st>>>(kp, s, ptc, t);
   } else {
     if (GF == 1) launch_nblist_tuned<false>(kp, s, ptc, t, st);
     else k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
@@ -2430,13 +2446,7 @@ cudaError_t launch_xfer_corr_lists(const KParams& kp, const Scratch& s, const zs
   if (cudaError_t e = reset_walls(s, st)) return e;
   k_xfer_classify<<<(kp.n + kSearchBlock - 1) / kSearchBlock, kSearchBlock, 0, st>>>(kp, s, t);
   mark(pf, "xfer_classify", st);
-  static int sms = 0;  // SMs of the device (the same for every B200)
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 148;
-  }
-  k_xfer_search<<<sms * 8, kSearchWarps * 32, 0, st>>>(kp, s, cur, t);
+  k_xfer_search<<<sm_count() * 8, kSearchWarps * 32, 0, st>>>(kp, s, cur, t);
   mark(pf, "xfer_search", st);
   k_nblist_xfer<<<(kp.n + kXferThreads - 1) / kXferThreads, kXferThreads, 0, st>>>(kp, s, cur, t);
   mark(pf, "nblist_xfer", st);
