@@ -419,6 +419,14 @@ __device__ __forceinline__ void append_walls(const KParams& kp, const Scratch& s
   if (wall && slot < kp.n) s.wl[slot] = i;
 }
 
+// Empties the wall list.  Every pass that may follow a list build or the wall
+// pass (boundary, governing, neighbour counts) does so in its first thread,
+// so that the next build finds it empty without a memory operation between
+// the kernels, which would also end their programmatic launch chain.
+__device__ __forceinline__ void empty_wall_list(const Scratch& s) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.misc[kMiscWalls] = 0;
+}
+
 // The end of particle i's list build, once s.nb holds its finished list
 // (cnt entries, or ovf): the particle's packed shadow record and list
 // count, and, for a non-fluid particle that can have a fluid neighbour in
@@ -699,6 +707,7 @@ template <int GF, int CW = kCellWarps, bool BATCH = false, bool PRECISE = false,
           bool SKIN = false>
 __global__ void __launch_bounds__(CW * 32, 42 / CW) k_nblist_seq(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
                                                                    zsph_tmp_t t) {
+  pdl_wait();
   const int wid = threadIdx.x >> 5;
   nblist_group<GF, CW, BATCH, PRECISE, SEGS, SKIN>(kp_arg, s, ptc, t, blockIdx.x * CW + wid, wid);
 }
@@ -719,6 +728,7 @@ constexpr int kSplitMax = 56000;
 template <bool BATCH, bool PRECISE>
 __global__ void __launch_bounds__(32 * kPlanes) k_nblist_split(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
                                                                zsph_tmp_t t) {
+  pdl_wait();
   constexpr int GF = 1, SEGS = kSegs;
   __shared__ __align__(16) float s_c[kPlanes][SEGS][3][kStage];
   __shared__ uint16_t s_e[kPlanes][32][kPlaneCap];
@@ -1051,6 +1061,7 @@ __device__ __forceinline__ void walls_block(const KParams& kp_arg, const Scratch
 
 template <int GF, bool PRECISE, bool BATCH, int LANES>
 __global__ void __launch_bounds__(kPairBlock, 8) k_walls(KParams kp, Scratch s, zsph_tmp_t t) {
+  pdl_wait();
   __shared__ int s_rs[kPairBlock / LANES * Stencil<GF>::NR];
   walls_block<GF, PRECISE, BATCH, false, LANES>(kp, s, t, nullptr, blockIdx.x, gridDim.x, threadIdx.x, s_rs);
 }
@@ -1167,6 +1178,8 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
 
 template <int GF, bool PRECISE = false, bool BATCH = false, bool REUSE = false>
 __global__ void __launch_bounds__(kPairBlock) k_boundary(KParams kp_arg, Scratch s, zsph_ptc_t ptc, zsph_tmp_t t) {
+  pdl_wait();
+  empty_wall_list(s);
   extern __shared__ __align__(16) unsigned char dsm[];
   boundary_one<GF, PRECISE, BATCH, REUSE>(kp_arg, s, ptc, t, blockIdx.x * kPairBlock + threadIdx.x,
                                           PairSmem<GF>(dsm), true);
@@ -1367,6 +1380,8 @@ template <int GF, int MODE, bool FEAT = false, bool PRECISE = false, bool BATCH 
           int MINB = 1, bool REUSE = false>
 __global__ void __launch_bounds__(kPairBlock, MINB)
     k_governing(KParams kp_arg, Scratch s, zsph_ptc_t ptc, zsph_tmp_t t, zsph_ptc_t out, FeatOut fo) {
+  pdl_wait();
+  empty_wall_list(s);
   extern __shared__ __align__(16) unsigned char dsm[];
   governing_one<GF, MODE, FEAT, PRECISE, BATCH, RIGID, REUSE>(kp_arg, s, ptc, t, out, fo,
                                                                blockIdx.x * kPairBlock + threadIdx.x,
@@ -1387,6 +1402,8 @@ struct NbS {  // simple boundary / governing
 template <int GF>
 __global__ void __launch_bounds__(kPairBlock) k_boundary_simple(KParams kp, Scratch s, zsph_ptc_t ptc,
                                                                 zsph_tmp_t t) {
+  pdl_wait();
+  empty_wall_list(s);
   extern __shared__ __align__(16) unsigned char dsm[];
   PairSmem<GF> sm(dsm);
   const int i = blockIdx.x * kPairBlock + threadIdx.x;
@@ -1420,6 +1437,8 @@ __global__ void __launch_bounds__(kPairBlock) k_boundary_simple(KParams kp, Scra
 template <int GF, int MODE>
 __global__ void __launch_bounds__(kPairBlock) k_governing_simple(KParams kp, Scratch s, zsph_ptc_t ptc,
                                                                  zsph_tmp_t t, zsph_ptc_t out) {
+  pdl_wait();
+  empty_wall_list(s);
   extern __shared__ __align__(16) unsigned char dsm[];
   PairSmem<GF> sm(dsm);
   const int i = blockIdx.x * kPairBlock + threadIdx.x;
@@ -1476,7 +1495,7 @@ template <bool BATCH>
 void launch_nblist_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc, const zsph_tmp_t& t,
                          cudaStream_t st) {
   if (kp.n <= kSplitMax) {
-    k_nblist_split<BATCH, false><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
+    launch_pdl(k_nblist_split<BATCH, false>, (kp.n + 31) / 32, 32 * kPlanes, 0, st, kp, s, ptc, t);
     return;
   }
   // (eight cells per CTA would exceed the 48 KB of static shared memory)
@@ -1485,13 +1504,13 @@ void launch_nblist_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
   const int segs = kp.tune_segs ? kp.tune_segs : kSegs;
   const int g4 = (kp.n + 127) / 128, g2 = (kp.n + 63) / 64;
   if (kp.tune_cw == 4) {
-    if (segs == 2) k_nblist_seq<1, 4, BATCH, false, 2><<<g4, 128, 0, st>>>(kp, s, ptc, t);
-    else if (segs == 3) k_nblist_seq<1, 4, BATCH, false, 3><<<g4, 128, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 4, BATCH, false, 4><<<g4, 128, 0, st>>>(kp, s, ptc, t);
+    if (segs == 2) launch_pdl(k_nblist_seq<1, 4, BATCH, false, 2>, g4, 128, 0, st, kp, s, ptc, t);
+    else if (segs == 3) launch_pdl(k_nblist_seq<1, 4, BATCH, false, 3>, g4, 128, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 4, BATCH, false, 4>, g4, 128, 0, st, kp, s, ptc, t);
   } else {
-    if (segs == 2) k_nblist_seq<1, 2, BATCH, false, 2><<<g2, 64, 0, st>>>(kp, s, ptc, t);
-    else if (segs == 3) k_nblist_seq<1, 2, BATCH, false, 3><<<g2, 64, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 2, BATCH, false, 4><<<g2, 64, 0, st>>>(kp, s, ptc, t);
+    if (segs == 2) launch_pdl(k_nblist_seq<1, 2, BATCH, false, 2>, g2, 64, 0, st, kp, s, ptc, t);
+    else if (segs == 3) launch_pdl(k_nblist_seq<1, 2, BATCH, false, 3>, g2, 64, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 2, BATCH, false, 4>, g2, 64, 0, st, kp, s, ptc, t);
   }
 }
 
@@ -1522,9 +1541,9 @@ void launch_governing_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_
   const FeatOut none{};
   const int nb = thread_blocks(kp.n), sm = pair_smem<1>(0, 0);
   switch (kp.tune_minb ? kp.tune_minb : BATCH ? 1 : governing_minb(kp.n)) {
-    case 6: k_governing<1, MODE, false, false, BATCH, false, 6><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
-    case 8: k_governing<1, MODE, false, false, BATCH, false, 8><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
-    default: k_governing<1, MODE, false, false, BATCH, false, 1><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none); break;
+    case 6: launch_pdl(k_governing<1, MODE, false, false, BATCH, false, 6>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none); break;
+    case 8: launch_pdl(k_governing<1, MODE, false, false, BATCH, false, 8>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none); break;
+    default: launch_pdl(k_governing<1, MODE, false, false, BATCH, false, 1>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none); break;
   }
 }
 
@@ -1536,50 +1555,43 @@ inline int walls_grid(int n, int lanes) {
 }
 template <int GF, bool PRECISE = false, bool BATCH = false>
 void launch_walls(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, cudaStream_t st) {
-  if (kp.n <= kWallsFew) k_walls<GF, PRECISE, BATCH, 8><<<walls_grid(kp.n, 8), kPairBlock, 0, st>>>(kp, s, t);
-  else k_walls<GF, PRECISE, BATCH, 2><<<walls_grid(kp.n, 2), kPairBlock, 0, st>>>(kp, s, t);
-}
-
-// zeroes the wall-list length before a list build appends to it
-inline cudaError_t reset_walls(const Scratch& s, cudaStream_t st) {
-  return cudaMemsetAsync(s.misc + kMiscWalls, 0, sizeof(int), st);
+  if (kp.n <= kWallsFew) launch_pdl(k_walls<GF, PRECISE, BATCH, 8>, walls_grid(kp.n, 8), kPairBlock, 0, st, kp, s, t);
+  else launch_pdl(k_walls<GF, PRECISE, BATCH, 2>, walls_grid(kp.n, 2), kPairBlock, 0, st, kp, s, t);
 }
 
 template <int GF>
 cudaError_t boundary_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc, const zsph_tmp_t& t,
                         cudaStream_t st, Prof* pf) {
-  if (cudaError_t e = reset_walls(s, st)) return e;
   if (kp.scenes) {  // batched form (grid factor 1, delta equations)
     if (GF != 1 || kp.equations != ZSPH_EQ_DELTA || kp.c3o) return cudaErrorInvalidValue;
     launch_nblist_tuned<true>(kp, s, ptc, t, st);
     mark(pf, "nblist", st);
     launch_walls<1, false, true>(kp, s, t, st);
     mark(pf, "walls", st);
-    k_boundary<1, false, true><<<thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st>>>(kp, s, ptc, t);
+    launch_pdl(k_boundary<1, false, true>, thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st, kp, s, ptc, t);
     mark(pf, "boundary", st);
     return cudaGetLastError();
   }
   if (kp.c3o) {  // precision form (grid factor 1, delta equations)
     if (GF != 1 || kp.equations != ZSPH_EQ_DELTA) return cudaErrorInvalidValue;
-    if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 2, false, true><<<(kp.n + 63) / 64, 64, 0, st>>>(kp, s, ptc, t);
+    if (kp.n <= kSplitMax) launch_pdl(k_nblist_split<false, true>, (kp.n + 31) / 32, 32 * kPlanes, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 2, false, true>, (kp.n + 63) / 64, 64, 0, st, kp, s, ptc, t);
     mark(pf, "nblist", st);
     launch_walls<1, true>(kp, s, t, st);
     mark(pf, "walls", st);
-    k_boundary<1, true><<<thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st>>>(kp, s, ptc, t);
+    launch_pdl(k_boundary<1, true>, thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st, kp, s, ptc, t);
     mark(pf, "boundary", st);
     return cudaGetLastError();
   }
   if (GF == 1) launch_nblist_tuned<false>(kp, s, ptc, t, st);
-  else k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
+  else launch_pdl(k_nblist_seq<GF, kSeqWarps<GF>>, (kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st, kp, s, ptc, t);
   mark(pf, "nblist", st);
   launch_walls<GF>(kp, s, t, st);
   mark(pf, "walls", st);
   if (kp.equations == ZSPH_EQ_SIMPLE)
-    k_boundary_simple<GF><<<thread_blocks(kp.n), kPairBlock, pair_smem<GF>(0, 0), st>>>(kp, s, ptc, t);
+    launch_pdl(k_boundary_simple<GF>, thread_blocks(kp.n), kPairBlock, pair_smem<GF>(0, 0), st, kp, s, ptc, t);
   else
-    k_boundary<GF><<<thread_blocks(kp.n), kPairBlock, pair_smem<GF>(kp.stage_windows ? 2 : 0, kWinCapB), st>>>(
-        kp, s, ptc, t);
+    launch_pdl(k_boundary<GF>, thread_blocks(kp.n), kPairBlock, pair_smem<GF>(kp.stage_windows ? 2 : 0, kWinCapB), st, kp, s, ptc, t);
   mark(pf, "boundary", st);
   return cudaGetLastError();
 }
@@ -1590,9 +1602,9 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
   const int nb = thread_blocks(kp.n);
   if (kp.equations == ZSPH_EQ_SIMPLE) {
     const int ss = pair_smem<GF>(0, 0);
-    if (mode == 0) k_governing_simple<GF, 0><<<nb, kPairBlock, ss, st>>>(kp, s, ptc, t, out);
-    if (mode == 1) k_governing_simple<GF, 1><<<nb, kPairBlock, ss, st>>>(kp, s, ptc, t, out);
-    if (mode == 2) k_governing_simple<GF, 2><<<nb, kPairBlock, ss, st>>>(kp, s, ptc, t, out);
+    if (mode == 0) launch_pdl(k_governing_simple<GF, 0>, nb, kPairBlock, ss, st, kp, s, ptc, t, out);
+    if (mode == 1) launch_pdl(k_governing_simple<GF, 1>, nb, kPairBlock, ss, st, kp, s, ptc, t, out);
+    if (mode == 2) launch_pdl(k_governing_simple<GF, 2>, nb, kPairBlock, ss, st, kp, s, ptc, t, out);
     mark(pf, "governing", st);
     return cudaGetLastError();
   }
@@ -1600,7 +1612,7 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     if (GF != 1 || feat || kp.c3o) return cudaErrorInvalidValue;
     const FeatOut none{};
     const int s1 = pair_smem<1>(0, 0);
-    if (mode == 0) k_governing<1, 0, false, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
+    if (mode == 0) launch_pdl(k_governing<1, 0, false, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     if (mode == 1) launch_governing_tuned<1, true>(kp, s, ptc, t, out, st);
     if (mode == 2) launch_governing_tuned<2, true>(kp, s, ptc, t, out, st);
     mark(pf, "governing", st);
@@ -1610,13 +1622,13 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     if (GF != 1 || feat) return cudaErrorInvalidValue;
     const FeatOut none{};
     const int s1 = pair_smem<1>(0, 0);
-    if (mode == 0) k_governing<1, 0, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
+    if (mode == 0) launch_pdl(k_governing<1, 0, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     if (kp.rigid_f) {  // floating body: also the fluid's force on its particles
-      if (mode == 1) k_governing<1, 1, false, true, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
-      if (mode == 2) k_governing<1, 2, false, true, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
+      if (mode == 1) launch_pdl(k_governing<1, 1, false, true, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+      if (mode == 2) launch_pdl(k_governing<1, 2, false, true, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     } else {
-      if (mode == 1) k_governing<1, 1, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
-      if (mode == 2) k_governing<1, 2, false, true><<<nb, kPairBlock, s1, st>>>(kp, s, ptc, t, out, none);
+      if (mode == 1) launch_pdl(k_governing<1, 1, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+      if (mode == 2) launch_pdl(k_governing<1, 2, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     }
     mark(pf, "governing", st);
     return cudaGetLastError();
@@ -1624,15 +1636,15 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
   const int sm = pair_smem<GF>(kp.stage_windows ? 3 : 0, kWinCapG);
   if (feat) {
     if (mode != 1) return cudaErrorInvalidValue;
-    k_governing<GF, 1, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, *feat);
+    launch_pdl(k_governing<GF, 1, true>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, *feat);
     mark(pf, "governing_feat", st);
     return cudaGetLastError();
   }
   const FeatOut none{};
   if (kp.rigid_f && mode != 0) {  // floating body, absolute positions
     if (GF != 1) return cudaErrorInvalidValue;
-    if (mode == 1) k_governing<1, 1, false, false, false, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none);
-    if (mode == 2) k_governing<1, 2, false, false, false, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none);
+    if (mode == 1) launch_pdl(k_governing<1, 1, false, false, false, true>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
+    if (mode == 2) launch_pdl(k_governing<1, 2, false, false, false, true>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
     mark(pf, "governing", st);
     return cudaGetLastError();
   }
@@ -1643,9 +1655,9 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     mark(pf, "governing", st);
     return cudaGetLastError();
   }
-  if (mode == 0) k_governing<GF, 0><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none);
-  if (mode == 1) k_governing<GF, 1><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none);
-  if (mode == 2) k_governing<GF, 2><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, out, none);
+  if (mode == 0) launch_pdl(k_governing<GF, 0>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
+  if (mode == 1) launch_pdl(k_governing<GF, 1>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
+  if (mode == 2) launch_pdl(k_governing<GF, 2>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
   mark(pf, "governing", st);
   return cudaGetLastError();
 }
@@ -1658,11 +1670,11 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
     launch_nblist_tuned<true>(kp, s, ptc, t, st);
   } else if (kp.c3o) {
     if (GF != 1) return cudaErrorInvalidValue;
-    if (kp.n <= kSplitMax) k_nblist_split<false, true><<<(kp.n + 31) / 32, 32 * kPlanes, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 2, false, true><<<(kp.n + 63) / 64, 64, 0, st>>>(kp, s, ptc, t);
+    if (kp.n <= kSplitMax) launch_pdl(k_nblist_split<false, true>, (kp.n + 31) / 32, 32 * kPlanes, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 2, false, true>, (kp.n + 63) / 64, 64, 0, st, kp, s, ptc, t);
   } else {
     if (GF == 1) launch_nblist_tuned<false>(kp, s, ptc, t, st);
-    else k_nblist_seq<GF, kSeqWarps<GF>><<<(kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st>>>(kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<GF, kSeqWarps<GF>>, (kp.n + 32 * kSeqWarps<GF> - 1) / (32 * kSeqWarps<GF>), kSeqWarps<GF> * 32, 0, st, kp, s, ptc, t);
   }
   return cudaGetLastError();
 }
@@ -1677,7 +1689,7 @@ cudaError_t nblist_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc
 //
 // k_cur_cells: each particle's y cell index at its current position, with
 // the hash's arithmetic (hash.cu:13); the non-fluid particles are appended to
-// s.wl (its length zeroed before).
+// s.wl (empty after the predictor's passes).
 __global__ void __launch_bounds__(kSearchBlock) k_cur_cells(KParams kp, Scratch s, zsph_ptc_t ptc, int* cy) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool act = i < kp.n;
@@ -1912,6 +1924,7 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_batch_persistent(Persist
       if (!grid_barrier(a)) return;
       persistent_pairs<0>(a, dsm);
       if (!grid_barrier(a)) return;
+      empty_wall_list(s);
       if (sub == 1) persistent_pairs<1>(a, dsm);
       else persistent_pairs<2>(a, dsm);
       if (!grid_barrier(a)) return;
@@ -1924,6 +1937,7 @@ __global__ void __launch_bounds__(kPersistThreads, 2) k_batch_persistent(Persist
 template <int GF>
 __global__ void __launch_bounds__(kSearchBlock) k_nb_counts(KParams kp, Scratch s, int* nb_boundary,
                                                             int* nb_governing) {
+  empty_wall_list(s);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kp.n) return;
   const int cnt = s.nb_cnt[i];
@@ -2360,15 +2374,14 @@ cudaError_t launch_corrector_reuse(const KParams& kp_in, const Scratch& s, const
   kp.cur_cy = cy;
   cudaError_t e = launch_pack_shadows(kp, s, ptc, st);
   if (e) return e;
-  if ((e = reset_walls(s, st))) return e;
   k_cur_cells<<<(kp.n + kSearchBlock - 1) / kSearchBlock, kSearchBlock, 0, st>>>(kp, s, ptc, cy);
   const int nb = thread_blocks(kp.n), sm = pair_smem<1>(0, 0);
   if (kp.n <= kWallsFew) k_walls_reuse<1, 8><<<walls_grid(kp.n, 8), kPairBlock, 0, st>>>(kp, s, ptc, t, fresh_boundary ? 0 : 1);
   else k_walls_reuse<1, 2><<<walls_grid(kp.n, 2), kPairBlock, 0, st>>>(kp, s, ptc, t, fresh_boundary ? 0 : 1);
-  if (fresh_boundary) k_boundary<1, false, false, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t);
+  if (fresh_boundary) launch_pdl(k_boundary<1, false, false, true>, nb, kPairBlock, sm, st, kp, s, ptc, t);
   const FeatOut none{};
-  if (mode == 2) k_governing<1, 2, false, false, false, false, 1, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, ptc, none);
-  else k_governing<1, 0, false, false, false, false, 1, true><<<nb, kPairBlock, sm, st>>>(kp, s, ptc, t, ptc, none);
+  if (mode == 2) launch_pdl(k_governing<1, 2, false, false, false, false, 1, true>, nb, kPairBlock, sm, st, kp, s, ptc, t, ptc, none);
+  else launch_pdl(k_governing<1, 0, false, false, false, false, 1, true>, nb, kPairBlock, sm, st, kp, s, ptc, t, ptc, none);
   return cudaGetLastError();
 }
 
@@ -2418,22 +2431,21 @@ cudaError_t launch_xfer_pred_lists(const KParams& kp, const Scratch& s, const zs
   if (kp.n == 0) return cudaSuccess;
   if (kp.p.grid_factor != 1 || kp.scenes || kp.c3o || kp.stage_windows || kp.equations != ZSPH_EQ_DELTA || !s.xf.sk)
     return cudaErrorInvalidValue;
-  if (cudaError_t e = reset_walls(s, st)) return e;
   const int segs = kp.tune_segs ? kp.tune_segs : kSegs;
   const int g4 = (kp.n + 127) / 128, g2 = (kp.n + 63) / 64;
   if (kp.tune_cw == 4) {
-    if (segs == 2) k_nblist_seq<1, 4, false, false, 2, true><<<g4, 128, 0, st>>>(kp, s, ptc, t);
-    else if (segs == 3) k_nblist_seq<1, 4, false, false, 3, true><<<g4, 128, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 4, false, false, 4, true><<<g4, 128, 0, st>>>(kp, s, ptc, t);
+    if (segs == 2) launch_pdl(k_nblist_seq<1, 4, false, false, 2, true>, g4, 128, 0, st, kp, s, ptc, t);
+    else if (segs == 3) launch_pdl(k_nblist_seq<1, 4, false, false, 3, true>, g4, 128, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 4, false, false, 4, true>, g4, 128, 0, st, kp, s, ptc, t);
   } else {
-    if (segs == 2) k_nblist_seq<1, 2, false, false, 2, true><<<g2, 64, 0, st>>>(kp, s, ptc, t);
-    else if (segs == 3) k_nblist_seq<1, 2, false, false, 3, true><<<g2, 64, 0, st>>>(kp, s, ptc, t);
-    else k_nblist_seq<1, 2, false, false, 4, true><<<g2, 64, 0, st>>>(kp, s, ptc, t);
+    if (segs == 2) launch_pdl(k_nblist_seq<1, 2, false, false, 2, true>, g2, 64, 0, st, kp, s, ptc, t);
+    else if (segs == 3) launch_pdl(k_nblist_seq<1, 2, false, false, 3, true>, g2, 64, 0, st, kp, s, ptc, t);
+    else launch_pdl(k_nblist_seq<1, 2, false, false, 4, true>, g2, 64, 0, st, kp, s, ptc, t);
   }
   mark(pf, "nblist", st);
   launch_walls<1>(kp, s, t, st);
   mark(pf, "walls", st);
-  k_boundary<1><<<thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st>>>(kp, s, ptc, t);
+  launch_pdl(k_boundary<1>, thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st, kp, s, ptc, t);
   mark(pf, "boundary", st);
   return cudaGetLastError();
 }
@@ -2443,7 +2455,6 @@ cudaError_t launch_xfer_corr_lists(const KParams& kp, const Scratch& s, const zs
   if (kp.n == 0) return cudaSuccess;
   if (kp.p.grid_factor != 1 || kp.scenes || kp.c3o || kp.stage_windows || kp.equations != ZSPH_EQ_DELTA || !s.xf.nb2)
     return cudaErrorInvalidValue;
-  if (cudaError_t e = reset_walls(s, st)) return e;
   k_xfer_classify<<<(kp.n + kSearchBlock - 1) / kSearchBlock, kSearchBlock, 0, st>>>(kp, s, t);
   mark(pf, "xfer_classify", st);
   k_xfer_search<<<sm_count() * 8, kSearchWarps * 32, 0, st>>>(kp, s, cur, t);
@@ -2467,7 +2478,7 @@ cudaError_t launch_xfer_corr_lists(const KParams& kp, const Scratch& s, const zs
   mark(pf, "nblist_fallback", st);
   launch_walls<1>(kp, s2, t, st);
   mark(pf, "walls", st);
-  k_boundary<1><<<thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st>>>(kp, s2, cur, t);
+  launch_pdl(k_boundary<1>, thread_blocks(kp.n), kPairBlock, pair_smem<1>(0, 0), st, kp, s2, cur, t);
   mark(pf, "boundary", st);
   return cudaGetLastError();
 }
