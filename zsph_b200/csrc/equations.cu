@@ -177,7 +177,7 @@ __device__ __forceinline__ void walk(const KParams& kp, const Scratch& s, int i,
         for (int e = 0; e < 4; ++e) nb[e] = fetch(js[h + e] >= 0 ? js[h + e] : fdummy);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (js[h + e] >= 0) use(nb[e]);
+          use(nb[e], js[h + e] >= 0);
       }
     }
     return;
@@ -188,7 +188,7 @@ __device__ __forceinline__ void walk(const KParams& kp, const Scratch& s, int i,
     for (int j = a; j < b; ++j) {
       if (j == i) continue;
       const float4 pj = shadow_pr<PRECISE>(kp, s, j, ci);
-      if (interacts(kp, dist2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z))) use(fetch(fb[r * kPairBlock] + (j - a)));
+      if (interacts(kp, dist2(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z))) use(fetch(fb[r * kPairBlock] + (j - a)), true);
     }
   }
 }
@@ -1099,8 +1099,10 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
   // a = 1 - q / 2; the products with x_ij are formed once (t) and shared by
   // the matrix, div v and the density sums.  The pass is bound by its
   // instructions as much as by the L1 data pipe: with frm multiplied into
-  // every term it took 1006 us at 4.2 M particles, 115 at 445 k and 22.7 at
-  // 20 k, now 924, 106 and 20.3.
+  // every term it took 1006 us at 4.2 M particles and 22.7 at 20 k, formed
+  // once 925 and 20.1.  A slot without a neighbour (another row, the list's
+  // end) fetches the particle itself and adds zeros: without a branch per
+  // neighbour the four chains overlap, 892 and 18.5 us.
   const float nh = -0.5f * kp.inv_h, cm = kp.c_fr * p.m;
   // The reference's second loop (delta_ns.cu:133-175) walks the same
   // neighbours with a constant matrix M: sum_j (M x_ij) f_j = M sum_j x_ij f_j,
@@ -1110,26 +1112,25 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
   float sx = 0.f, sy = 0.f, sz = 0.f;
   // reused lists: the boundary rows by the current cells (the lists' rows are the cells at build time)
   const int cy_i = REUSE ? kp.cur_cy[i] : 0;
-  auto use1 = [&](const auto& nb) {
+  auto use1 = [&](const auto& nb, bool ok) {
     const float dx = pi.x - nb.pr.x, dy = pi.y - nb.pr.y, dz = pi.z - nb.pr.z;
     if constexpr (REUSE) {
-      if (!interacts(kp, dist2(dx, dy, dz))) return;
+      if (!ok || !interacts(kp, dist2(dx, dy, dz))) return;
       const int row = nb.cy - cy_i;
       if (row < -GF || row >= GF) return;
     }
     const float a = __fmaf_rn(sqrt_fast(dist2(dx, dy, dz)), nh, 1.0f);
     const float r1 = fabsf(nb.pr.w);
-    const float frm = a * a * a * (cm * rcp_fast(r1));
+    const float frm = ok ? a * a * a * (cm * rcp_fast(r1)) : 0.0f;
     const float tx = dx * frm, ty = dy * frm, tz = dz * frm;
     Lxx = __fmaf_rn(-dx, tx, Lxx); Lxy = __fmaf_rn(-dx, ty, Lxy); Lxz = __fmaf_rn(-dx, tz, Lxz);
     Lyy = __fmaf_rn(-dy, ty, Lyy); Lyz = __fmaf_rn(-dy, tz, Lyz); Lzz = __fmaf_rn(-dz, tz, Lzz);
     const float dr = r1 - rho_self;  // delta_ns.cu:163-164
     sx = __fmaf_rn(dr, tx, sx); sy = __fmaf_rn(dr, ty, sy); sz = __fmaf_rn(dr, tz, sz);
-    if (fi && fluid_of(nb.pr.w)) {
-      divv = __fmaf_rn(nb.vp.x - vi.x, tx, divv);
-      divv = __fmaf_rn(nb.vp.y - vi.y, ty, divv);
-      divv = __fmaf_rn(nb.vp.z - vi.z, tz, divv);
-    }
+    float dv = (nb.vp.x - vi.x) * tx;
+    dv = __fmaf_rn(nb.vp.y - vi.y, ty, dv);
+    dv = __fmaf_rn(nb.vp.z - vi.z, tz, dv);
+    divv += ok && fi && fluid_of(nb.pr.w) ? dv : 0.0f;
   };
   const float4* win = sm.win;
   if constexpr (REUSE) {  // every list entry, classified by the current cells in use1
@@ -1141,7 +1142,10 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
   } else {
     if (staged)
       walk<GF, true, NbB1>(kp, s, i, pi, sm.rs, sm.re, sm.fb, 0, kWinCapB - 1,
-                           [&](int q) { return NbB1{win[2 * q], win[2 * q + 1]}; }, use1);
+                           [&](int q) { return NbB1{win[2 * q], win[2 * q + 1]}; },
+                           [&](const NbB1& nb, bool ok) {
+                             if (ok) use1(nb, true);  // the dummy is another particle here
+                           });
     else
       walk<GF, true, NbB1, PRECISE>(kp, s, i, pi, sm.rs, sm.re, sm.rs, i, kp.n - 1,
                                     [&](int q) {
@@ -1266,7 +1270,8 @@ __device__ __forceinline__ void governing_one(const KParams& kp_arg, const Scrat
   FeatAcc fa;
   const bool rig = RIGID && ptc.type[i] == 2;
   float3 rf = make_float3(0.f, 0.f, 0.f);
-  auto use = [&](const NbG& nb) {
+  auto use = [&](const NbG& nb, bool ok) {
+    if (!ok) return;
     const float dx = pi.x - nb.pr.x, dy = pi.y - nb.pr.y, dz = pi.z - nb.pr.z;
     const float rr2 = dist2(dx, dy, dz);
     if constexpr (REUSE) {
@@ -1421,8 +1426,8 @@ __global__ void __launch_bounds__(kPairBlock) k_boundary_simple(KParams kp, Scra
           const ShadowRec r = s.sh.load(q);
           return NbB1{r.pr, r.vp};
         },
-        [&](const NbB1& nb) {
-          if (!fluid_of(nb.pr.w)) return;
+        [&](const NbB1& nb, bool ok) {
+          if (!ok || !fluid_of(nb.pr.w)) return;
           const float dx = pi.x - nb.pr.x, dy = pi.y - nb.pr.y, dz = pi.z - nb.pr.z;
           const float a = __fmaf_rn(sqrt_fast(dist2(dx, dy, dz)), nh, 1.0f);
           const float dvdx = (vi.x - nb.vp.x) * dx + (vi.y - nb.vp.y) * dy + (vi.z - nb.vp.z) * dz;
@@ -1456,7 +1461,8 @@ __global__ void __launch_bounds__(kPairBlock) k_governing_simple(KParams kp, Scr
         const ShadowRec r = s.sh.load(q);
         return NbS{r.pr, r.vp, t.dofv[q]};
       },
-      [&](const NbS& nb) {
+      [&](const NbS& nb, bool ok) {
+        if (!ok) return;
         const float dx = pi.x - nb.pr.x, dy = pi.y - nb.pr.y, dz = pi.z - nb.pr.z;
         const float rr2 = dist2(dx, dy, dz);
         const float dvdx = (vi.x - nb.vp.x) * dx + (vi.y - nb.vp.y) * dy + (vi.z - nb.vp.z) * dz;
