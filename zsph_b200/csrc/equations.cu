@@ -485,8 +485,8 @@ constexpr int kCellWarps = 4;  // warps per CTA in the list build
 //
 // The walls' (rho, p) come after, from the finished lists (k_walls).
 // list build: hit words queued per lane (a power of two, more than 7; less with many warps' shared memory)
-// the 5x5 stencil's rows leave up to 25 words, and a drain halfway finds only the round's lanes full
-template <int GF, int CW> constexpr int kQueueOf = GF == 2 ? 16 : CW > 4 ? 8 : 16;
+// (5x5 stencil at 153 k particles: 555 us with 8 words, 570 with 16, 646 with 32)
+template <int GF, int CW> constexpr int kQueueOf = GF == 2 ? 8 : CW > 4 ? 8 : 16;
 constexpr int kSegs = 4;   // list build: cells whose lanes test their own rows concurrently
 constexpr int kStage = 66; // list build: staged candidates per segment (64) plus two floats of padding
 // warps per CTA of k_nblist_seq (the 5x5 stencil's row starts need more shared memory)
