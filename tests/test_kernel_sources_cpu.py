@@ -1,0 +1,52 @@
+"""Ordering rules of the kernels that no run can show reliably, checked in
+their sources: what a kernel reads must stay behind the wait for the kernel
+that wrote it."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "zsph_b200", "csrc")
+SOURCES = {os.path.basename(p): re.sub(r"//[^\n]*", "", open(p).read())
+           for p in sorted(glob.glob(os.path.join(CSRC, "*.cu*")))}
+
+
+def _body(text, start):
+    """The brace block that opens first at or after `start`."""
+    a = text.index("{", start)
+    depth = 0
+    for k in range(a, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[k], 0)
+        if depth == 0:
+            return text[a + 1:k]
+    raise AssertionError("unbalanced braces")
+
+
+def _kernels():
+    """name -> body of every __global__ function."""
+    out = {}
+    for text in SOURCES.values():
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s+)?(\w+)\s*\(", text):
+            out[m.group(1)] = _body(text, text.index(")", m.end()))
+    return out
+
+
+def test_inline_loads_are_volatile():
+    """An asm load that is not volatile may move above griddepcontrol.wait or a grid barrier."""
+    for name, text in SOURCES.items():
+        for m in re.finditer(r"\basm\s*(volatile)?\s*\(", text):
+            statement = text[m.start():text.index(";\n", m.end())]
+            if re.search(r"\b(ld|ldmatrix|red|atom)\.", statement):
+                assert m.group(1), (name, statement[:80])
+
+
+def test_programmatic_kernels_wait_first():
+    """A kernel launched while its predecessor drains touches no memory before pdl_wait()."""
+    launched = set()
+    for text in SOURCES.values():
+        for m in re.finditer(r"\blaunch_pdl\(([^;]*?);", text):
+            launched |= set(re.findall(r"\bk_\w+", m.group(1)))
+    kernels = _kernels()
+    assert len(launched) >= 10 and launched <= set(kernels)
+    for name in launched:
+        first = [s.strip() for s in kernels[name].split(";") if not s.strip().startswith("__shared__")][0]
+        assert first == "pdl_wait()", (name, first)

@@ -124,18 +124,22 @@ __host__ __device__ __forceinline__ int3 unpack_cell(int c) {
 }
 
 // 256-bit global load / store of one 32-byte record (sm_100 v8 vector
-// access; the address must be 32-byte aligned).
+// access; the address must be 32-byte aligned).  The loads are volatile: an
+// asm statement that is not counts as a function of its operands, which a
+// compiler may move above pdl_wait() or a grid barrier (a particle's own
+// record's address is known before either), or merge with a load on the
+// other side of one.
 __device__ __forceinline__ void ld_rec(const float4* p, float4& a, float4& b) {
-  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
 }
 // ld_rec where `ok`; elsewhere no access is made and a, b are undefined.
 __device__ __forceinline__ void ld_rec_if(bool ok, const float4* p, float4& a, float4& b) {
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
-      "@p ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p), "r"((unsigned)ok));
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
+               "@p ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p), "r"((unsigned)ok));
 }
 __device__ __forceinline__ void st_rec(float4* p, float4 a, float4 b) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
