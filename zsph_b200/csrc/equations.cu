@@ -485,9 +485,17 @@ constexpr int kCellWarps = 4;  // warps per CTA in the list build
 //
 // The walls' (rho, p) come after, from the finished lists (k_walls).
 // list build: hit words queued per lane (a power of two, more than 7; less with many warps' shared memory)
-// (5x5 stencil at 153 k particles: 555 us with 8 words, 570 with 16, 646 with 32)
+// (5x5 stencil at 153 k particles, four segments: 555 us with 8 words, 570 with 16, 646 with 32)
 template <int GF, int CW> constexpr int kQueueOf = GF == 2 ? 8 : CW > 4 ? 8 : 16;
 constexpr int kSegs = 4;   // list build: cells whose lanes test their own rows concurrently
+// The 5x5 stencil's cells hold a few particles each (side h), so a group of 32
+// spans some 15 cells.  With four segments it took four rounds, and a full
+// queue was drained with a quarter of the lanes at work: 256 / 302 / 368 / 520 us
+// at 40 / 105 / 152 / 242 k particles, 1360 at 844 k (227 / 277 / 351 / 505 and
+// 1335 when every row's hits were emitted at once).  Eight segments, two
+// rounds: 159 / 193 / 256 / 361 and 1006.  Sixteen fill the shared memory:
+// 122 / 197 / 252 / 368 and 1123.
+template <int GF> constexpr int kSegsOf = GF == 2 ? 8 : kSegs;
 constexpr int kStage = 66; // list build: staged candidates per segment (64) plus two floats of padding
 // warps per CTA of k_nblist_seq (the 5x5 stencil's row starts need more shared memory)
 template <int GF> constexpr int kSeqWarps = GF == 1 ? kCellWarps : 2;
@@ -704,9 +712,9 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
   }
 }
 
-template <int GF, int CW = kCellWarps, bool BATCH = false, bool PRECISE = false, int SEGS = kSegs,
+template <int GF, int CW = kCellWarps, bool BATCH = false, bool PRECISE = false, int SEGS = kSegsOf<GF>,
           bool SKIN = false>
-__global__ void __launch_bounds__(CW * 32, 42 / CW) k_nblist_seq(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
+__global__ void __launch_bounds__(CW * 32, GF == 2 ? 26 / CW : 42 / CW) k_nblist_seq(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
                                                                    zsph_tmp_t t) {
   pdl_wait();
   const int wid = threadIdx.x >> 5;
@@ -911,7 +919,10 @@ template <int GF> struct PairSmem {
 // shuffles: one thread, 8 and 2 lanes take 74, 110 and 72 us at 4.2 M, 70, 90
 // and 64 us for 24 scenes of 0.98 M together.  Hence 8 lanes up to kWallsFew
 // particles, 2 beyond.  Eight resident CTAs (64 registers): 2 lanes took
-// 83 us at 4.2 M with 80.
+// 83 us at 4.2 M with 80.  The 5x5 stencil's lists hold the neighbours of 25
+// rows, of which a wall uses 20: 4 lanes at every size, 10 / 20 / 31 / 73 us at
+// 13 / 105 / 242 / 844 k particles, against 10 / 23 / 39 / 105 with 8,
+// 17 / 22 / 35 / 75 with 2 and 27 / 29 / 34 / 73 with one thread and one sum.
 constexpr int kWallsFew = 300000;
 
 // This thread's partial sums of wall i (lane q of its LANES lanes).  rs: row
@@ -1564,7 +1575,8 @@ inline int walls_grid(int n, int lanes) {
 }
 template <int GF, bool PRECISE = false, bool BATCH = false>
 void launch_walls(const KParams& kp, const Scratch& s, const zsph_tmp_t& t, cudaStream_t st) {
-  if (kp.n <= kWallsFew) launch_pdl(k_walls<GF, PRECISE, BATCH, 8>, walls_grid(kp.n, 8), kPairBlock, 0, st, kp, s, t);
+  if constexpr (GF != 1) launch_pdl(k_walls<GF, PRECISE, BATCH, 4>, walls_grid(kp.n, 4), kPairBlock, 0, st, kp, s, t);
+  else if (kp.n <= kWallsFew) launch_pdl(k_walls<GF, PRECISE, BATCH, 8>, walls_grid(kp.n, 8), kPairBlock, 0, st, kp, s, t);
   else launch_pdl(k_walls<GF, PRECISE, BATCH, 2>, walls_grid(kp.n, 2), kPairBlock, 0, st, kp, s, t);
 }
 
