@@ -1547,7 +1547,9 @@ inline int sm_count() {
 // Register budget of the plain governing pass when none was tuned: at 93
 // registers five CTAs fit an SM, at 80 six.  A case whose CTAs fit the device
 // at once with six but leave a nearly empty second wave with five (94,720 to
-// 113,664 particles on 148 SMs) takes six: 48.8 against 53.5 us at 105 k.
+// 113,664 particles on 148 SMs) takes six: 48.8 against 53.5 us at 105 k, and
+// 46.6 against 50.7 with the 5x5 stencil (96 registers), whose other sizes are
+// faster or equal without it.
 inline int governing_minb(int n) {
   const int ctas = thread_blocks(n), sms = sm_count();
   return ctas > 5 * sms && ctas <= 6 * sms ? 6 : 1;
@@ -1673,6 +1675,13 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     if (mode == 0) launch_governing_tuned<0, false>(kp, s, ptc, t, out, st);
     if (mode == 1) launch_governing_tuned<1, false>(kp, s, ptc, t, out, st);
     if (mode == 2) launch_governing_tuned<2, false>(kp, s, ptc, t, out, st);
+    mark(pf, "governing", st);
+    return cudaGetLastError();
+  }
+  if (GF != 1 && governing_minb(kp.n) == 6) {
+    if (mode == 0) launch_pdl(k_governing<GF, 0, false, false, false, false, 6>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
+    if (mode == 1) launch_pdl(k_governing<GF, 1, false, false, false, false, 6>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
+    if (mode == 2) launch_pdl(k_governing<GF, 2, false, false, false, false, 6>, nb, kPairBlock, sm, st, kp, s, ptc, t, out, none);
     mark(pf, "governing", st);
     return cudaGetLastError();
   }
