@@ -542,9 +542,16 @@ __device__ __forceinline__ void hits32(const float* sx, u64 px, u64 py, u64 pz, 
   if constexpr (SKIN) mk <<= (32 - n) & 31;
 }
 
-// At least 42 warps per SM (a register budget of 40-48 without spills in the
-// plain form, 9.9 KB of shared memory per 2-warp CTA): the kernel is
-// issue-bound and hides its staging loads with more resident warps.
+// The kernel is issue-bound and hides its staging loads with other resident
+// warps: as many CTAs per SM as their staging arrays and queues leave room for
+// in its 228 KB (1 KB of each CTA's is the system's) -- 15 of two warps with
+// four segments, 14.5 KB each -- and the registers that those leave (64, no
+// spills).  Asking for 42 warps (40 registers, spills of 8 and 16 bytes in the
+// precision and batched forms) brought none more and cost 308 against 300 us
+// per step at 105 k particles, 7649 / 7524 at 4.2 M, 1925 / 1870 for 24 scenes
+// and 945 / 926 with a floating body at 362 k.
+template <int GF, int CW, int SEGS>
+constexpr int kListCtas = 228 * 1024 / (CW * (SEGS * 3 * kStage * 4 + kQueueOf<GF, CW> * 32 * 8) + 1024);
 //
 // nblist_group is the work of one warp on group `group` (particles
 // 32*group .. 32*group+31); k_nblist_seq runs one group per warp, the
@@ -714,7 +721,7 @@ __device__ __forceinline__ void nblist_group(const KParams& kp_arg, const Scratc
 
 template <int GF, int CW = kCellWarps, bool BATCH = false, bool PRECISE = false, int SEGS = kSegsOf<GF>,
           bool SKIN = false>
-__global__ void __launch_bounds__(CW * 32, GF == 2 ? 26 / CW : 42 / CW) k_nblist_seq(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
+__global__ void __launch_bounds__(CW * 32, kListCtas<GF, CW, SEGS>) k_nblist_seq(KParams kp_arg, Scratch s, zsph_ptc_t ptc,
                                                                    zsph_tmp_t t) {
   pdl_wait();
   const int wid = threadIdx.x >> 5;
@@ -857,7 +864,7 @@ __global__ void __launch_bounds__(32 * kPlanes) k_nblist_split(KParams kp_arg, S
 // only when the transfer's conditions failed this step (*s.xf.flag set);
 // otherwise every CTA returns at once.
 template <int CW, int SEGS>
-__global__ void __launch_bounds__(CW * 32, 42 / CW) k_nblist_fallback(KParams kp, Scratch s, zsph_ptc_t ptc,
+__global__ void __launch_bounds__(CW * 32, kListCtas<1, CW, SEGS>) k_nblist_fallback(KParams kp, Scratch s, zsph_ptc_t ptc,
                                                                         zsph_tmp_t t) {
   if (*s.xf.flag == 0) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(s.xf.stats + 1, 1ull);
