@@ -1577,9 +1577,12 @@ inline int sm_count() {
 // 113,664 particles on 148 SMs) takes six: 48.8 against 53.5 us at 105 k, and
 // 46.6 against 50.7 with the 5x5 stencil (96 registers), whose other sizes are
 // faster or equal without it.
-inline int governing_minb(int n) {
+// The precision form (`fit` = 4 CTAs at 110 registers) likewise: 43.5 / 52.1 /
+// 58.4 us at 79 / 96 / 114 k with six, 46.6 / 54.2 / 61.6 without; a floating body
+// in it gains at 85 k and loses as much at 114 k, and keeps the compiler's.
+inline int governing_minb(int n, int fit = 5) {
   const int ctas = thread_blocks(n), sms = sm_count();
-  return ctas > 5 * sms && ctas <= 6 * sms ? 6 : 1;
+  return ctas > fit * sms && ctas <= 6 * sms ? 6 : 1;
 }
 
 // governing (grid factor 1, no shared-memory windows) with the tuned register
@@ -1672,10 +1675,15 @@ cudaError_t governing_gf(const KParams& kp, const Scratch& s, const zsph_ptc_t& 
     if (GF != 1 || feat) return cudaErrorInvalidValue;
     const FeatOut none{};
     const int s1 = pair_smem<1>(0, 0);
-    if (mode == 0) launch_pdl(k_governing<1, 0, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+    const bool six = governing_minb(kp.n, 4) == 6;  // 110 registers: four CTAs
+    if (mode == 0 && six) launch_pdl(k_governing<1, 0, false, true, false, false, 6>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+    else if (mode == 0) launch_pdl(k_governing<1, 0, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     if (kp.rigid_f) {  // floating body: also the fluid's force on its particles
       if (mode == 1) launch_pdl(k_governing<1, 1, false, true, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
       if (mode == 2) launch_pdl(k_governing<1, 2, false, true, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+    } else if (six) {
+      if (mode == 1) launch_pdl(k_governing<1, 1, false, true, false, false, 6>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
+      if (mode == 2) launch_pdl(k_governing<1, 2, false, true, false, false, 6>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
     } else {
       if (mode == 1) launch_pdl(k_governing<1, 1, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
       if (mode == 2) launch_pdl(k_governing<1, 2, false, true>, nb, kPairBlock, s1, st, kp, s, ptc, t, out, none);
