@@ -1121,7 +1121,9 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
   // every term it took 1006 us at 4.2 M particles and 22.7 at 20 k, formed
   // once 925 and 20.1.  A slot without a neighbour (another row, the list's
   // end) fetches the particle itself and adds zeros: without a branch per
-  // neighbour the four chains overlap, 892 and 18.5 us.
+  // neighbour the four chains overlap, 892 and 18.5 us.  A particle whose own
+  // densities' difference is not finite takes a walk of its own (below), with
+  // the branch; a select in every slot instead took 15.0 against 13.5 us.
   const float nh = -0.5f * kp.inv_h, cm = kp.c_fr * p.m;
   // The reference's second loop (delta_ns.cu:133-175) walks the same
   // neighbours with a constant matrix M: sum_j (M x_ij) f_j = M sum_j x_ij f_j,
@@ -1187,6 +1189,15 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
                            [&](const NbB1& nb, bool ok) {
                              if (ok) use1(nb, true);  // the dummy is another particle here
                            });
+    else if (GF == 1 && !isfinite(fabsf(pi.w) - rho_self))  // an empty slot's zero times this is not zero
+      walk<GF, true, NbB1, PRECISE>(kp, s, i, pi, sm.rs, sm.re, sm.rs, i, kp.n - 1,
+                                    [&](int q) {
+                                      const ShadowRec r = shadow_rec<PRECISE>(kp, s, q, ci);
+                                      return NbB1{r.pr, r.vp};
+                                    },
+                                    [&](const NbB1& nb, bool ok) {
+                                      if (ok) use1(nb, true);
+                                    }, ci);
     else
       walk<GF, true, NbB1, PRECISE>(kp, s, i, pi, sm.rs, sm.re, sm.rs, i, kp.n - 1,
                                     [&](int q) {
