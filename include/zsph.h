@@ -541,24 +541,32 @@ int zsph_persistent_barrier_test(zsph_handle_t* h, int spin_limit, void* stream)
  * (warps) per CTA of the neighbour-list build {2, 4}, cells (segments) a
  * list-build warp handles together per round {2, 3, 4}, minimum resident
  * CTAs per SM of the governing kernel {1, 6, 8} (its register budget), steps
- * per graph replay of zsph_run {1, 4} (36 candidates) -- for trial_steps steps each on the
- * handle's buffers, restores old_ and the carried tmp arrays after every
- * trial, and keeps the fastest for the handle's later zsph_run calls. */
+ * per graph replay of zsph_run {1, 4} (36 candidates) -- and the untuned
+ * shapes (below; with 1 and 4 steps per graph, not counted as candidates) for
+ * trial_steps steps each on the handle's buffers, restores old_ and the
+ * carried tmp arrays after every trial, and keeps the fastest for the handle's
+ * later zsph_run calls: a field of the result is 0 where the untuned shapes
+ * were the fastest.
+ * Untuned (0), the list build takes 2 warps per CTA and 4 segments, and up to
+ * 56,000 particles a form of its own with three warps per 32 particles, one
+ * per plane of the stencil; the governing pass takes the compiler's registers
+ * (1), or 6 CTAs per SM where six hold all of a single case's CTAs at once and
+ * five do not (94,720 < n <= 113,664 on 148 SMs); 1 step per graph.
+ * Either list field set to a candidate turns the small form off. */
 typedef struct {
   int list_cells_per_cta, governing_min_ctas, steps_per_graph;
   float ms_per_step;  /* of the chosen shapes */
   float ms_default;   /* of the untuned shapes */
   int candidates;
-  int list_segments;  /* list build: cells handled together per round {2, 3, 4} (0: the default, 4) */
+  int list_segments;  /* list build: cells handled together per round {2, 3, 4} (0: the default) */
 } zsph_tune_t;
 int zsph_autotune(zsph_handle_t* h, const zsph_ptc_t* old_, const zsph_ptc_t* new_, const zsph_tmp_t* tmp,
                   int trial_steps, zsph_tune_t* out, void* stream);
 /* Applies launch shapes chosen earlier (a zsph_autotune result kept by the
  * caller, e.g. across restarts of the same case) without timing anything:
  * list_cells_per_cta, list_segments, governing_min_ctas and steps_per_graph
- * from the candidate sets above, 0 for each one's default (2 warps, 4
- * segments, 1 CTA, 1 step); the time fields are ignored.  ZSPH_EINVAL for any
- * other value. */
+ * from the candidate sets above, 0 for each one's default (the untuned shape
+ * above); the time fields are ignored.  ZSPH_EINVAL for any other value. */
 int zsph_set_launch_shapes(zsph_handle_t* h, const zsph_tune_t* shapes);
 
 /* ---- Precision form (no reference counterpart) ----------------------------

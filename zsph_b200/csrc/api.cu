@@ -718,7 +718,15 @@ int zsph_autotune(zsph_handle_t* h, const zsph_ptc_t* o, const zsph_ptc_t* w, co
     }
     return cudaSuccess;
   };
-  const int cws[] = {2, 4}, segss[] = {2, 3, 4}, minbs[] = {1, 6, 8}, spgs[] = {1, 4};
+  // the untuned shapes first (0: the defaults, which depend on the particle
+  // count), so that they stay unless a candidate is faster
+  struct Shape { int cw, sg, mb, spg; };
+  std::vector<Shape> shapes{{0, 0, 0, 1}, {0, 0, 0, 4}};
+  const size_t untuned = shapes.size();
+  for (int cw : {2, 4})
+    for (int sg : {2, 3, 4})
+      for (int mb : {1, 6, 8})
+        for (int spg : {1, 4}) shapes.push_back({cw, sg, mb, spg});
   zsph_tune_t best{};
   best.ms_per_step = 1e30f;
   float ms_default = 0.f;
@@ -729,40 +737,39 @@ int zsph_autotune(zsph_handle_t* h, const zsph_ptc_t* o, const zsph_ptc_t* w, co
   cudaError_t e = copy(true);
   if (!e) e = cudaEventCreate(&e0);
   if (!e) e = cudaEventCreate(&e1);
-  for (int cw : cws)
-    for (int sg : segss)
-    for (int mb : minbs)
-      for (int spg : spgs) {
-        if (e) break;
-        h->kp.tune_cw = cw;
-        h->kp.tune_segs = sg;
-        h->kp.tune_minb = mb;
-        h->graph_steps = spg;
-        if (h->graph) {
-          cudaGraphExecDestroy(h->graph);
-          h->graph = nullptr;
-        }
-        e = copy(false);
-        if (!e && zsph_run(h, o, w, tmp, spg, stream) != ZSPH_OK) e = cudaErrorUnknown;  // capture + warm-up
-        const int launches = (trial_steps + spg - 1) / spg;
-        if (!e) e = cudaEventRecord(e0, st);
-        if (!e && zsph_run(h, o, w, tmp, launches * spg, stream) != ZSPH_OK) e = cudaErrorUnknown;
-        if (!e) e = cudaEventRecord(e1, st);
-        if (!e) e = cudaEventSynchronize(e1);
-        float ms = 0.f;
-        if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
-        if (e) break;
-        ms /= (float)(launches * spg);
-        ++count;
-        if (cw == 2 && sg == 4 && mb == 1 && spg == 1) ms_default = ms;  // the untuned shapes
-        if (ms < best.ms_per_step) {
-          best.ms_per_step = ms;
-          best.list_cells_per_cta = cw;
-          best.list_segments = sg;
-          best.governing_min_ctas = mb;
-          best.steps_per_graph = spg;
-        }
-      }
+  for (size_t k = 0; k < shapes.size() && !e; ++k) {
+    const Shape& sh = shapes[k];
+    h->kp.tune_cw = sh.cw;
+    h->kp.tune_segs = sh.sg;
+    h->kp.tune_minb = sh.mb;
+    h->graph_steps = sh.spg;
+    if (h->graph) {
+      cudaGraphExecDestroy(h->graph);
+      h->graph = nullptr;
+    }
+    e = copy(false);
+    const int warm = sh.spg + (k ? 0 : trial_steps);  // capture + warm-up, longer for the first
+    if (!e && zsph_run(h, o, w, tmp, warm, stream) != ZSPH_OK) e = cudaErrorUnknown;
+    if (!e && !k) e = copy(false);
+    const int launches = (trial_steps + sh.spg - 1) / sh.spg;
+    if (!e) e = cudaEventRecord(e0, st);
+    if (!e && zsph_run(h, o, w, tmp, launches * sh.spg, stream) != ZSPH_OK) e = cudaErrorUnknown;
+    if (!e) e = cudaEventRecord(e1, st);
+    if (!e) e = cudaEventSynchronize(e1);
+    float ms = 0.f;
+    if (!e) e = cudaEventElapsedTime(&ms, e0, e1);
+    if (e) break;
+    ms /= (float)(launches * sh.spg);
+    if (k >= untuned) ++count;
+    if (k == 0) ms_default = ms;
+    if (ms < best.ms_per_step) {
+      best.ms_per_step = ms;
+      best.list_cells_per_cta = sh.cw;
+      best.list_segments = sh.sg;
+      best.governing_min_ctas = sh.mb;
+      best.steps_per_graph = sh.spg;
+    }
+  }
   if (h->graph) {
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;

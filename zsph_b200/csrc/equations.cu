@@ -1547,12 +1547,12 @@ __global__ void __launch_bounds__(kSearchBlock) k_integrate(KParams kp, zsph_ptc
 
 inline int thread_blocks(int n) { return (n + kPairBlock - 1) / kPairBlock; }
 
-// list build (grid factor 1): a plane per warp for small cases, else with the
-// tuned number of cells per CTA
+// list build (grid factor 1): with the tuned shapes where any were set, else a
+// plane per warp for small cases
 template <bool BATCH>
 void launch_nblist_tuned(const KParams& kp, const Scratch& s, const zsph_ptc_t& ptc, const zsph_tmp_t& t,
                          cudaStream_t st) {
-  if (kp.n <= kSplitMax) {
+  if (kp.n <= kSplitMax && !kp.tune_cw && !kp.tune_segs) {
     launch_pdl(k_nblist_split<BATCH, false>, (kp.n + 31) / 32, 32 * kPlanes, 0, st, kp, s, ptc, t);
     return;
   }
