@@ -50,3 +50,17 @@ def test_programmatic_kernels_wait_first():
     for name in launched:
         first = [s.strip() for s in kernels[name].split(";") if not s.strip().startswith("__shared__")][0]
         assert first == "pdl_wait()", (name, first)
+
+
+def test_every_search_empties_the_wall_list():
+    """A step that ended between a list build and the pass after it (a bounded
+    barrier that ran out) leaves wall-list entries behind, which must not reach
+    the lists of a new order; no call can be made to end there, so the sources
+    are read: the last kernel of either search empties the list, as the
+    persistent step does, and the wall pass leaves fluid records alone."""
+    kernels = _kernels()
+    for name in ("k_rank_gather", "k_gather_by_index", "k_batch_persistent"):
+        assert re.search(r"misc\[kMiscWalls\]\s*=\s*0;", kernels[name]), name
+    text = SOURCES["equations.cu"]
+    body = _body(text, text.index("void walls_block("))
+    assert "fluid_of(own.pr.w)" in body[:body.index("wall_sums<")]

@@ -422,7 +422,9 @@ __device__ __forceinline__ void append_walls(const KParams& kp, const Scratch& s
 // Empties the wall list.  Every pass that may follow a list build or the wall
 // pass (boundary, governing, neighbour counts) does so in its first thread,
 // so that the next build finds it empty without a memory operation between
-// the kernels, which would also end their programmatic launch chain.
+// the kernels, which would also end their programmatic launch chain.  A step
+// cut off in between (a bounded barrier that ran out) leaves entries behind:
+// the searches empty the list too, before any list of the new order is built.
 __device__ __forceinline__ void empty_wall_list(const Scratch& s) {
   if (blockIdx.x == 0 && threadIdx.x == 0) s.misc[kMiscWalls] = 0;
 }
@@ -1062,10 +1064,11 @@ __device__ __forceinline__ void walls_block(const KParams& kp_arg, const Scratch
       }
     }
     if (LANES > 1) __syncwarp();
-    if (act) wall_sums<GF, PRECISE, CY, LANES>(kp, s, t, i, q, rs, W, own.pr, rsum, wsum);
+    const bool wall = act && !fluid_of(own.pr.w);  // never a fluid record, whatever the list holds
+    if (wall) wall_sums<GF, PRECISE, CY, LANES>(kp, s, t, i, q, rs, W, own.pr, rsum, wsum);
     float rt = wall_tree<LANES>(rsum);
     const float wt = wall_tree<LANES>(wsum);
-    if (!act || q != 0) continue;
+    if (!wall || q != 0) continue;
     const zsph_gpu_param_t& p = kp.p;
     if (fabsf(wt) > 1e-8f) rt = rt / wt; else rt = 0.0f;
     if (rt < 0.0f) rt = 0.0f;

@@ -251,7 +251,10 @@ __global__ void __launch_bounds__(kSearchBlock, 8) k_rank_gather(KParams kp, Scr
                                                                  zsph_tmp_t t) {
   pdl_wait();
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot == 0) sc.misc[kMiscFluidEpoch] = sc.misc[6];  // this search's cell stamps are valid
+  if (slot == 0) {
+    sc.misc[kMiscFluidEpoch] = sc.misc[6];  // this search's cell stamps are valid
+    sc.misc[kMiscWalls] = 0;                // whatever an interrupted step left
+  }
   if (slot >= kp.n) return;
   rank_gather_one(kp, sc, o, w, t, slot);
 }
@@ -271,7 +274,10 @@ __global__ void __launch_bounds__(kSearchBlock) k_rank_values(KParams kp, Scratc
 __global__ void __launch_bounds__(kSearchBlock) k_gather_by_index(KParams kp, Scratch sc, zsph_ptc_t o,
                                                                   zsph_ptc_t w, zsph_tmp_t t) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot == 0) sc.misc[kMiscFluidEpoch] = 0;  // no cell stamps for this sort: the wall pass takes every wall
+  if (slot == 0) {
+    sc.misc[kMiscFluidEpoch] = 0;  // no cell stamps for this sort: the wall pass takes every wall
+    sc.misc[kMiscWalls] = 0;       // whatever an interrupted step left
+  }
   if (slot >= kp.n) return;
   gather_one(o, w, t.index[slot], slot);
 }

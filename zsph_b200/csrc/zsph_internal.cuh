@@ -250,7 +250,7 @@ struct Scratch {
   int* misc;         // [kMiscWords] 0: tiles done, 1: last key, 2: count of last key, 3: big-cell list length,
                      //       4: largest key (one-pass scan), 5: one-pass scan tile counter, 6: one-pass scan epoch,
                      //       7: the fused scatter's finished-CTA counter (crowded cells),
-                     //       kMiscWalls: entries in wl (zeroed by the passes that follow a list build),
+                     //       kMiscWalls: entries in wl (zeroed by the searches and by the passes that follow a list build),
                      //       kMiscFluidEpoch: the epoch of the cfe stamps (0 after the drop-in gather)
   unsigned long long* tile_state;  // [tiles] one-pass scan: (tag << 32) | prefix value, tag from the epoch
   int* big_list;     // [kBigListCap]
