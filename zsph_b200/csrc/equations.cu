@@ -478,7 +478,8 @@ constexpr int kCellWarps = 4;  // warps per CTA in the list build
 // candidates as it was tested (a loop as long as the fullest lane's hits in
 // it, into a ring) cost 2.5 times the iterations: 1446 against 1220 us at
 // 4.2 M particles, 62.7 against 54.5 at 105 k; with queues of 8 words instead
-// of 16 (less shared memory, more drains) 1251 and 57.2.
+// of 16 (less shared memory, more drains) 1251 and 57.2.  (1070 and 49 with the
+// tests and the registers below.)
 //
 // Precision form: candidates are moved into the frame of the lane's own
 // cell (its position is the offset from that cell's corner, as in the pair
@@ -544,16 +545,17 @@ __device__ __forceinline__ void hits32(const float* sx, u64 px, u64 py, u64 pz, 
   if constexpr (SKIN) mk <<= (32 - n) & 31;
 }
 
-// The kernel is issue-bound and hides its staging loads with other resident
-// warps: as many CTAs per SM as their staging arrays and queues leave room for
-// in its 228 KB (1 KB of each CTA's is the system's) -- 15 of two warps with
-// four segments, 14.5 KB each -- and the registers that those leave (64, no
+// The kernel is issue-bound (75 % issue-active at 1.4 M particles) and hides
+// its staging loads with other resident warps: as many CTAs per SM as their
+// staging arrays and queues leave room for in its 228 KB (in units of 128
+// bytes, 1 KB of each CTA's the system's) -- 14 of two warps with four
+// segments, 14.5 KB each -- and the registers that those leave (72, no
 // spills).  Asking for 42 warps (40 registers, spills of 8 and 16 bytes in the
-// precision and batched forms) brought none more and cost 308 against 300 us
-// per step at 105 k particles, 7649 / 7524 at 4.2 M, 1925 / 1870 for 24 scenes
-// and 945 / 926 with a floating body at 362 k.
+// precision and batched forms) brought none more and cost 307.5 against
+// 298.3 us per step at 105 k particles, 7650 / 7519 at 4.2 M, 1925 / 1874 for
+// 24 scenes and 945 / 926 with a floating body at 362 k.
 template <int GF, int CW, int SEGS>
-constexpr int kListCtas = 228 * 1024 / (CW * (SEGS * 3 * kStage * 4 + kQueueOf<GF, CW> * 32 * 8) + 1024);
+constexpr int kListCtas = 228 * 1024 / ((CW * (SEGS * 3 * kStage * 4 + kQueueOf<GF, CW> * 32 * 8) + 127) / 128 * 128 + 1024);
 //
 // nblist_group is the work of one warp on group `group` (particles
 // 32*group .. 32*group+31); k_nblist_seq runs one group per warp, the
@@ -735,10 +737,10 @@ __global__ void __launch_bounds__(CW * 32, kListCtas<GF, CW, SEGS>) k_nblist_seq
 // (row bounds, staging, tests, emission, row after row) is a third as long.
 // Each warp collects its plane's entries per lane in shared memory; the
 // planes' entries in order are the list, so it equals k_nblist_seq's entry
-// for entry.  13 k / 20 k / 34 k / 54 k particles: 21 / 24 / 31 / 36 us, against
-// 35 / 37 / 43 / 44 with one warp per group; equal at 61 k, and slower from
-// 105 k on (68 against 53), where warps are plenty and the planes' buffers
-// limit how many are resident.
+// for entry.  20 k / 34 k / 48 k / 54 k particles: 24 / 32 / 38 / 36 us, against
+// 33 / 39 / 39 / 41 with one warp per group; slower from 61 k on (47 against 43,
+// 51 / 46 at 81 k, 68 / 49 at 105 k), where warps are plenty and the planes'
+// buffers limit how many are resident.
 constexpr int kPlanes = 3;
 constexpr int kPlaneCap = kMaxNb + 2;  // 65 words per lane: the lanes' k-th entries fall in different banks
 constexpr int kSplitMax = 56000;
@@ -927,7 +929,8 @@ template <int GF> struct PairSmem {
 // walls it is bound by the instructions, to which lanes add row starts and
 // shuffles: one thread, 8 and 2 lanes take 74, 110 and 72 us at 4.2 M, 70, 90
 // and 64 us for 24 scenes of 0.98 M together.  Hence 8 lanes up to kWallsFew
-// particles, 2 beyond.  Eight resident CTAs (64 registers): 2 lanes took
+// particles, 2 beyond (equal at 290 k, 18.3 us; 22 against 19 at 348 k, 28 / 22
+// at 567 k).  Eight resident CTAs (64 registers): 2 lanes took
 // 83 us at 4.2 M with 80.  The 5x5 stencil's lists hold the neighbours of 25
 // rows, of which a wall uses 20: 4 lanes at every size, 10 / 20 / 31 / 73 us at
 // 13 / 105 / 242 / 844 k particles, against 10 / 23 / 39 / 105 with 8,
@@ -1119,10 +1122,11 @@ __device__ __forceinline__ void boundary_one(const KParams& kp_arg, const Scratc
   const float rho_self = reinterpret_cast<const float2*>(ptc.rhop)[i].x;  // old own density
   // The pair terms: frm = m / rho_j * (grad W / r) = cm a^3 / rho_j with
   // a = 1 - q / 2; the products with x_ij are formed once (t) and shared by
-  // the matrix, div v and the density sums.  The pass is bound by its
-  // instructions as much as by the L1 data pipe: with frm multiplied into
-  // every term it took 1006 us at 4.2 M particles and 22.7 at 20 k, formed
-  // once 925 and 20.1.  A slot without a neighbour (another row, the list's
+  // the matrix, div v and the density sums.  The pass is bound by the L1 data
+  // pipe (93 % of its wavefronts at 1.4 M particles, 62 % issue-active) and, when
+  // small, by the chain of its instructions: with frm multiplied into every
+  // term it took 1006 us at 4.2 M particles and 22.7 at 20 k, formed once 925
+  // and 20.1.  A slot without a neighbour (another row, the list's
   // end) fetches the particle itself and adds zeros: without a branch per
   // neighbour the four chains overlap, 892 and 18.5 us.  A particle whose own
   // densities' difference is not finite takes a walk of its own (below), with
@@ -1590,7 +1594,9 @@ inline int sm_count() {
 // at once with six but leave a nearly empty second wave with five (94,720 to
 // 113,664 particles on 148 SMs) takes six: 48.8 against 53.5 us at 105 k, and
 // 46.6 against 50.7 with the 5x5 stencil (96 registers), whose other sizes are
-// faster or equal without it.
+// faster or equal without it.  Not where six save one wave of several: the
+// drop-in pass with six / five took 93 / 81 us at 203 k (two waves, three), 93 /
+// 86 at 217 k, 107 / 95 at 242 k, 140 / 128 at 348 k.
 // The precision form (`fit` = 4 CTAs at 110 registers) likewise: 43.5 / 52.1 /
 // 58.4 us at 79 / 96 / 114 k with six, 46.6 / 54.2 / 61.6 without; a floating body
 // in it gains at 85 k and loses as much at 114 k, and keeps the compiler's.
