@@ -1,9 +1,11 @@
-"""Ordering rules of the kernels that no run can show reliably, checked in
-their sources: what a kernel reads must stay behind the wait for the kernel
-that wrote it."""
+"""Rules of the kernels that no run can show reliably, checked in their
+sources and in the compiler's report: what a kernel reads must stay behind the
+wait for the kernel that wrote it, and dispatch rules count the CTAs that fit."""
 import glob
 import os
 import re
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "zsph_b200", "csrc")
 SOURCES = {os.path.basename(p): re.sub(r"//[^\n]*", "", open(p).read())
@@ -64,3 +66,24 @@ def test_every_search_empties_the_wall_list():
     text = SOURCES["equations.cu"]
     body = _body(text, text.index("void walls_block("))
     assert "fluid_of(own.pr.w)" in body[:body.index("wall_sums<")]
+
+
+def test_governing_budgets_fit_the_dispatch_rule():
+    """The rule that takes six CTAs per SM counts five of the plain and the 5x5
+    pass at the compiler's registers, and four of the precision form's: the
+    build's own report must bear that out."""
+    report = os.path.join(CSRC, "..", "_build", "equations.cu.o.ptxas.txt")
+    if not os.path.exists(report):
+        pytest.skip("no compiler report (the library was built elsewhere)")
+    text = open(report).read()
+    regs = {m.group(1): int(m.group(2)) for m in
+            re.finditer(r"Compiling entry function '\w*k_governingI(\w+?)EEv\w*'.*?Used (\d+) registers", text, re.S)}
+
+    def ctas(gf, mode, precise, minb):
+        key = f"Li{gf}ELi{mode}ELb0ELb{precise}ELb0ELb0ELi{minb}ELb0E"
+        return 65536 // (128 * -(-regs[key] // 8) * 8)
+
+    for mode in (0, 1, 2):
+        for gf, precise, fit in ((1, 0, 5), (2, 0, 5), (1, 1, 4)):
+            assert ctas(gf, mode, precise, 1) == fit, (gf, mode, precise)
+            assert ctas(gf, mode, precise, 6) == 6, (gf, mode, precise)
